@@ -27,6 +27,9 @@
 namespace gk_fast {
 int fastmath_check(int n, unsigned long long seed, double* host_worst3);
 }
+namespace gk_parity {
+int math_eval(int n, const double* a, const double* b, double* out);
+}
 
 namespace gk {
 
@@ -236,6 +239,7 @@ int build_ctx(gk_handle* h) {
     ph.gm1Rec1 = ph.gm1Rec + 1.0;
     ph.gcq = ph.gamma * ph.cq;
     ph.hgm1 = 0.5 * ph.gm1;
+    ph.ranged = pd.gamma < 1024.0 && ph.gm1Rec < 1048576.0;
     ph.cfl = pd.cfl;
     ph.dmin = pd.dfloor;
     ph.pmin = pd.pfloor;
@@ -322,24 +326,18 @@ int env_int(const char* name, int dflt) {
 }
 
 // Tile shape of the fused 2D stage (threads per CTA, rows per tile), from the
-// grid: enough tiles for every resident CTA slot (148 SMs x 512/threads), at
+// grid: enough tiles for every resident CTA slot (148 SMs x stage_ctas), at
 // most 24 rows.  Each tile repeats a 4-row prologue, so longer tiles do less
 // work; but few waves of tiles leave a tail, and a small grid needs short
 // tiles and narrow CTAs for every SM to get work.  Measured:
-//   KH 4096^2, 128 threads, G zone-updates/s at 16 / 24 / 32 rows: fast
-//   17.6 / 17.8 / 17.8, parity 7.37 / 7.40 / 7.31;
-//   RT 1024x3072 (9 strips), same: fast 9.10 / 9.10 / 9.04, parity 4.09 /
-//   4.01 / 3.45 (1.5 waves at 32 rows);
-//   KH 256^2, us per step, 128 threads x 4 rows -> 64 x 2: fast 24.2 -> 20.7,
-//   parity 52.8 -> 38.3; KH 512^2, 128 x 4 -> 64 x 4: fast 37.9 -> 33.4,
-//   parity 92.7 -> 63.4.
-// Parity mode's heavier cells want more waves of long tiles where a grid has
-// more than one wave at 24 rows: it then aims at 4 waves with at least 12
-// rows.  Parity, us per step at the rows chosen (12 / 16 / 24 rows):
-// RT 1024x3072 761 (761 / 772 / 788), KH 2048^2 621 at 15 (625 / 631 / 666),
-// KH 4096^2 2267 at 24.  Smaller grids keep the one-wave rule, which a tail
-// wave would cost more than short tiles save: KH 1024^2 at 16 rows is one
-// wave of 576 tiles, 189 us (12 rows: 234).
+//   KH 4096^2 fast, 128 threads, G zone-updates/s at 16 / 24 / 32 rows:
+//   17.6 / 17.8 / 17.8; RT 1024x3072 (9 strips), same: 9.10 / 9.10 / 9.04;
+//   KH 256^2 fast, us per step, 128 threads x 4 rows -> 64 x 2: 24.2 -> 20.7;
+//   KH 512^2, 128 x 4 -> 64 x 4: 37.9 -> 33.4.
+// Parity mode's heavier cells want more waves of tiles where a grid has more
+// than one wave at 24 rows: it then aims at 4 waves with at least 12 rows.
+// Parity, us per step at 8 / 12 / 16 / 20 / 24 rows: KH 2001x1503 357 / 352 /
+// 341 / 347 / 365 (15 rows chosen).
 // GK_STAGE_THREADS / GK_STAGE_ROWS override (tuning).
 int stage_threads_for(const gk::Geom& g) {
     const int v = env_int("GK_STAGE_THREADS", 0);
@@ -376,7 +374,8 @@ int stage_rows(const gk::Geom& g, int threads, bool parity) {
     if (forced > 0) return forced;
     const long long cols = threads - 4;
     const long long strips = (g.nx + cols - 1) / cols;
-    const long long tiles = (long long)g.ny * strips, slots = 148LL * (512 / threads);
+    const long long tiles = (long long)g.ny * strips;
+    const long long slots = 148LL * gk::stage_ctas(threads, parity);
     const long long per_slot = (tiles + slots - 1) / slots;
     if (!parity || per_slot <= 24) return (int)std::max(2LL, std::min(24LL, per_slot));
     return (int)std::max(12LL, std::min(24LL, (tiles + 4 * slots - 1) / (4 * slots)));
@@ -1215,6 +1214,11 @@ int gk_checked_report(unsigned long long* count, unsigned long long* first) {
 int gk_fastmath_check(int n, unsigned long long seed, double* worst3) {
     if (n <= 0 || !worst3) return GK_ERR_INVALID;
     return gk_fast::fastmath_check(n, seed, worst3) == 0 ? GK_OK : GK_ERR_CUDA;
+}
+
+int gk_paritymath_eval(int n, const double* a, const double* b, double* out) {
+    if (n <= 0 || !a || !b || !out) return GK_ERR_INVALID;
+    return gk_parity::math_eval(n, a, b, out) == 0 ? GK_OK : GK_ERR_CUDA;
 }
 
 

@@ -26,6 +26,15 @@ inline bool first_on_device(std::atomic<unsigned long long>& mask) {
     return (mask.fetch_or(bit) & bit) == 0;
 }
 
+// Resident CTAs per SM the fused 2D stage is compiled for at nt threads per
+// CTA.  Fast mode: 512 threads at up to 128 registers.  Parity mode: 384 at
+// up to 168, so that the two Riemann problems of a row interleave without
+// spills (KH 2001x1503, us per step: 393 at 512 threads, 353 at 384 with the
+// same code); CTAs of 256 stay at two.
+constexpr int stage_ctas(int nt, bool parity) {
+    return parity && nt < 256 ? 384 / nt : 512 / nt;
+}
+
 // Device variable slots.
 enum Slot { S_DEN = 0, S_MTX = 1, S_MTY = 2, S_ENG = 3, S_MTZ = 4 };
 // Primitive slots use the same positions: rho, vx, vy, p, vz.
@@ -65,6 +74,8 @@ struct Phys {
     double gm1Rec1;                        // gm1Rec + 1: fast mode's E + p = p*gm1Rec1 + rho k/2
     double gcq;                            // gamma*cq: fast mode's gamma X = gamma p + gcq max(p* - p, 0)
     double hgm1;                           // (gamma-1)/2: fast mode's conversion
+    int ranged;                            // gamma in the range parity mode's branch-free
+                                           // division is built for (gk_physics.cuh)
     double cfl, dmin, pmin;
     double grav[3];
     int has_grav;

@@ -251,17 +251,36 @@ __global__ void k_immersed(double* __restrict__ u, Geom g, Phys ph, const DevTim
 
 // ------------------------------------------------------------ ConsToPrim
 // EquationOfState::ConsToPrim (adiabatic.cpp:18-61) over every stored cell.
+// denInv = 1/max(d, dmin)
 __device__ __forceinline__ void cons_to_prim5(double d, double mx, double my, double mz, double e,
-                                              const Phys& ph, double w[5]) {
+                                              double denInv, const Phys& ph, double w[5]) {
     d = GK_FLOOR(d, ph.dmin);
     w[gk::P_RHO] = d;
-    double denInv = GK_RCP(d);
     w[gk::P_VX] = mx * denInv;
     w[gk::P_VY] = my * denInv;
     w[gk::P_VZ] = mz * denInv;
     double engKin = 0.5 * denInv * (mx * mx + my * my + mz * mz);
     double pre = ph.gm1 * (e - engKin);
     w[gk::P_PRE] = GK_BELOW(ph.pmin, pre) ? pre : ph.pmin;
+}
+__device__ __forceinline__ void cons_to_prim5(double d, double mx, double my, double mz, double e,
+                                              const Phys& ph, double w[5]) {
+    cons_to_prim5(d, mx, my, mz, e, GK_RCP(GK_FLOOR(d, ph.dmin)), ph, w);
+}
+
+// Half van Leer slopes of five variables in cell b between cells a and c.
+__device__ __forceinline__ void half_slopes5(const double (&a)[5], const double (&b)[5],
+                                             const double (&c)[5], double (&h)[5]) {
+    SlopeRange r;
+    clear(r);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) h[v] = vanleer_half(b[v] - a[v], c[v] - b[v], r);
+#if !GK_FASTMATH
+    if (out_of_range(r)) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) h[v] = vanleer_half_any(b[v] - a[v], c[v] - b[v]);
+    }
+#endif
 }
 
 // EquationOfState::ConsToPrim (adiabatic.cpp:18-61) of every stored cell,
@@ -297,33 +316,36 @@ __global__ void k_flux(const double* __restrict__ w, double* __restrict__ F, Geo
     else if (dir == 1) { i = g.ib + a; j = g.jb + bidx; k = g.kb + cidx; if (i >= g.ie) return; }
     else { i = g.ib + a; j = g.jb + bidx; k = g.kb + cidx; if (i >= g.ie) return; }
     // cells m (left of the face) and p (right); stencil offsets
-    double wl[5], wr[5];
+    double l1[5], l2[5], l3[5], r1[5], r2[5], r3[5], wl[5], wr[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        double l1, l2, l3, r1, r2, r3;
         const double* p = w + v * g.vstride;
         if (dir == 0) {
-            l1 = p[sidx(g, k, j, i - 2)]; l2 = p[sidx(g, k, j, i - 1)]; l3 = p[sidx(g, k, j, i)];
-            r1 = l2; r2 = l3; r3 = p[sidx(g, k, j, i + 1)];
+            l1[v] = p[sidx(g, k, j, i - 2)]; l2[v] = p[sidx(g, k, j, i - 1)]; l3[v] = p[sidx(g, k, j, i)];
+            r1[v] = l2[v]; r2[v] = l3[v]; r3[v] = p[sidx(g, k, j, i + 1)];
         } else if (dir == 1) {
-            l1 = p[sidx(g, k, j - 2, i)]; l2 = p[sidx(g, k, j - 1, i)]; l3 = p[sidx(g, k, j, i)];
-            r1 = l2; r2 = l3; r3 = p[sidx(g, k, j + 1, i)];
+            l1[v] = p[sidx(g, k, j - 2, i)]; l2[v] = p[sidx(g, k, j - 1, i)]; l3[v] = p[sidx(g, k, j, i)];
+            r1[v] = l2[v]; r2[v] = l3[v]; r3[v] = p[sidx(g, k, j + 1, i)];
         } else {
-            l1 = p[sidx(g, k - 1, j - 1, i)]; l2 = p[sidx(g, k - 1, j, i)];
-            l3 = p[sidx(g, k - 1, j + 1, i)];
-            r1 = p[sidx(g, k, j - 1, i)]; r2 = p[sidx(g, k, j, i)]; r3 = p[sidx(g, k, j + 1, i)];
+            l1[v] = p[sidx(g, k - 1, j - 1, i)]; l2[v] = p[sidx(g, k - 1, j, i)];
+            l3[v] = p[sidx(g, k - 1, j + 1, i)];
+            r1[v] = p[sidx(g, k, j - 1, i)]; r2[v] = p[sidx(g, k, j, i)]; r3[v] = p[sidx(g, k, j + 1, i)];
         }
-        if (ph.plm) {
-#if GK_FASTMATH
-            wl[v] = l2 + vanleer_half(l2 - l1, l3 - l2);
-            wr[v] = r2 - vanleer_half(r2 - r1, r3 - r2);
-#else
-            wl[v] = l2 + 0.5 * vanleer(l2 - l1, l3 - l2);
-            wr[v] = r2 - 0.5 * vanleer(r2 - r1, r3 - r2);
-#endif
-        } else {
-            wl[v] = l2;
-            wr[v] = r2;
+    }
+    if (ph.plm) {
+        double hl[5], hr[5];
+        half_slopes5(l1, l2, l3, hl);
+        half_slopes5(r1, r2, r3, hr);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            wl[v] = l2[v] + hl[v];
+            wr[v] = r2[v] - hr[v];
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            wl[v] = l2[v];
+            wr[v] = r2[v];
         }
     }
     // rotation (hllc.cpp:25-27): x (vx | vy, vz), y (vy | vz, vx), z (vz | vx, vy)
@@ -698,23 +720,23 @@ __global__ void __launch_bounds__(1024) k_run1d(double* A, double* B, Geom g, Ph
         __syncthreads();
         if (t < nf) {
             const int i = g.ib + t;  // the face between cells i-1 and i
-            double wl[5], wr[5];
+            double l1[5], l2[5], r2[5], r3[5], wl[5], wr[5];
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
                 const double* p = W + v * g.lenx;
-                const double l1 = p[i - 2], l2 = p[i - 1], l3 = p[i];
-                const double r1 = l2, r2 = l3, r3 = p[i + 1];
-                if (ph.plm) {
-#if GK_FASTMATH
-                    wl[v] = l2 + vanleer_half(l2 - l1, l3 - l2);
-                    wr[v] = r2 - vanleer_half(r2 - r1, r3 - r2);
-#else
-                    wl[v] = l2 + 0.5 * vanleer(l2 - l1, l3 - l2);
-                    wr[v] = r2 - 0.5 * vanleer(r2 - r1, r3 - r2);
-#endif
-                } else {
-                    wl[v] = l2;
-                    wr[v] = r2;
+                l1[v] = p[i - 2];
+                l2[v] = wl[v] = p[i - 1];
+                r2[v] = wr[v] = p[i];
+                r3[v] = p[i + 1];
+            }
+            if (ph.plm) {
+                double hl[5], hr[5];
+                half_slopes5(l1, l2, r2, hl);
+                half_slopes5(l2, r2, r3, hr);
+#pragma unroll
+                for (int v = 0; v < 5; ++v) {
+                    wl[v] = l2[v] + hl[v];
+                    wr[v] = r2[v] - hr[v];
                 }
             }
             Flux5 f;
@@ -847,11 +869,9 @@ struct Q4 {
     double d, mx, my, e;
 };
 
-__device__ __forceinline__ W4 c2p4(const Q4& q, const Phys& ph) {
+__device__ __forceinline__ W4 c2p4(const Q4& q, double denInv, const Phys& ph) {
     W4 w;
-    double d = GK_FLOOR(q.d, ph.dmin);
-    w.r = d;
-    double denInv = GK_RCP(d);
+    w.r = GK_FLOOR(q.d, ph.dmin);
     w.vx = q.mx * denInv;
     w.vy = q.my * denInv;
 #if GK_FASTMATH
@@ -865,14 +885,39 @@ __device__ __forceinline__ W4 c2p4(const Q4& q, const Phys& ph) {
     return w;
 }
 
-#if GK_FASTMATH
-// Fast mode: vl4 returns half slopes and the face states add them directly.
-__device__ __forceinline__ W4 vl4(const W4& a, const W4& b, const W4& c) {
+// c2p4 with the reciprocal of the floored density: `bad` set where it is out
+// of range (parity mode), or of any state.
+__device__ __forceinline__ W4 c2p4(const Q4& q, const Phys& ph, bool& bad) {
+    return c2p4(q, rcp_ranged(GK_FLOOR(q.d, ph.dmin), bad), ph);
+}
+__device__ __forceinline__ W4 c2p4(const Q4& q, const Phys& ph) {
+    return c2p4(q, GK_RCP(GK_FLOOR(q.d, ph.dmin)), ph);
+}
+
+// Half van Leer slopes of cell b; the face states add them directly.
+__device__ __forceinline__ W4 vl4(const W4& a, const W4& b, const W4& c, SlopeRange& rg) {
     W4 s;
-    s.r = vanleer_half(b.r - a.r, c.r - b.r);
-    s.vx = vanleer_half(b.vx - a.vx, c.vx - b.vx);
-    s.vy = vanleer_half(b.vy - a.vy, c.vy - b.vy);
-    s.p = vanleer_half(b.p - a.p, c.p - b.p);
+    s.r = vanleer_half(b.r - a.r, c.r - b.r, rg);
+    s.vx = vanleer_half(b.vx - a.vx, c.vx - b.vx, rg);
+    s.vy = vanleer_half(b.vy - a.vy, c.vy - b.vy, rg);
+    s.p = vanleer_half(b.p - a.p, c.p - b.p, rg);
+    return s;
+}
+__device__ __forceinline__ W4 vl4_any(const W4& a, const W4& b, const W4& c) {
+    W4 s;
+    s.r = vanleer_half_any(b.r - a.r, c.r - b.r);
+    s.vx = vanleer_half_any(b.vx - a.vx, c.vx - b.vx);
+    s.vy = vanleer_half_any(b.vy - a.vy, c.vy - b.vy);
+    s.p = vanleer_half_any(b.p - a.p, c.p - b.p);
+    return s;
+}
+__device__ __forceinline__ W4 vl4(const W4& a, const W4& b, const W4& c) {
+    SlopeRange rg;
+    clear(rg);
+    W4 s = vl4(a, b, c, rg);
+#if !GK_FASTMATH
+    if (out_of_range(rg)) s = vl4_any(a, b, c);
+#endif
     return s;
 }
 __device__ __forceinline__ W4 plus_half(const W4& u, const W4& h) {
@@ -881,22 +926,6 @@ __device__ __forceinline__ W4 plus_half(const W4& u, const W4& h) {
 __device__ __forceinline__ W4 minus_half(const W4& u, const W4& h) {
     return W4{u.r - h.r, u.vx - h.vx, u.vy - h.vy, u.p - h.p};
 }
-#else
-__device__ __forceinline__ W4 vl4(const W4& a, const W4& b, const W4& c) {
-    W4 s;
-    s.r = vanleer(b.r - a.r, c.r - b.r);
-    s.vx = vanleer(b.vx - a.vx, c.vx - b.vx);
-    s.vy = vanleer(b.vy - a.vy, c.vy - b.vy);
-    s.p = vanleer(b.p - a.p, c.p - b.p);
-    return s;
-}
-__device__ __forceinline__ W4 plus_half(const W4& u, const W4& s) {
-    return W4{u.r + 0.5 * s.r, u.vx + 0.5 * s.vx, u.vy + 0.5 * s.vy, u.p + 0.5 * s.p};
-}
-__device__ __forceinline__ W4 minus_half(const W4& u, const W4& s) {
-    return W4{u.r - 0.5 * s.r, u.vx - 0.5 * s.vx, u.vy - 0.5 * s.vy, u.p - 0.5 * s.p};
-}
-#endif
 
 __device__ __forceinline__ Q4 ldq(const double* __restrict__ u, long long vs, long long c) {
     return Q4{__ldg(u + c), __ldg(u + vs + c), __ldg(u + 2 * vs + c), __ldg(u + 3 * vs + c)};
@@ -906,9 +935,26 @@ __device__ __forceinline__ Q4 ldq(const double* __restrict__ u, long long vs, lo
 __device__ __forceinline__ void hllc_y(const W4& l, const W4& r, const Phys& ph, Flux5& f) {
     hllc<false, kSel>(l.r, l.vy, l.vx, 0.0, l.p, r.r, r.vy, r.vx, 0.0, r.p, ph, f);
 }
-// x face: rotation (vx | vy, vz).
-__device__ __forceinline__ void hllc_x(const W4& l, const W4& r, const Phys& ph, Flux5& f) {
-    hllc<false, kSel>(l.r, l.vx, l.vy, 0.0, l.p, r.r, r.vx, r.vy, 0.0, r.p, ph, f);
+// The x face (rotation (vx | vy, vz)) and the y face of a row, solved
+// together: both Riemann problems are straight-line code, so their
+// instruction streams interleave; in parity mode one test then completes the
+// few lanes whose states are out of range.
+__device__ __forceinline__ void hllc_xy(const W4& xl, const W4& xr, Flux5& fx, const W4& yl,
+                                        const W4& yr, Flux5& fy, const Phys& ph) {
+    bool badx = !ph.ranged, bady = !ph.ranged;
+    HllcAux ax, ay;
+    hllc_ranged<false, kSel>(xl.r, xl.vx, xl.vy, 0.0, xl.p, xr.r, xr.vx, xr.vy, 0.0, xr.p, ph, fx,
+                             badx, ax);
+    hllc_ranged<false, kSel>(yl.r, yl.vy, yl.vx, 0.0, yl.p, yr.r, yr.vy, yr.vx, 0.0, yr.p, ph, fy,
+                             bady, ay);
+#if !GK_FASTMATH
+    if (badx || bady || ax.zero || ay.zero) {
+        hllc_redo<false, kSel>(xl.r, xl.vx, xl.vy, 0.0, xl.p, xr.r, xr.vx, xr.vy, 0.0, xr.p, ph, fx,
+                               badx, ax);
+        hllc_redo<false, kSel>(yl.r, yl.vy, yl.vx, 0.0, yl.p, yr.r, yr.vy, yr.vx, 0.0, yr.p, ph, fy,
+                               bady, ay);
+    }
+#endif
 }
 
 // KIND 0: u' = c1*uc - c2*dF (stage 1); 1: u' = c1*u0 + c2*uc - c3*dF
@@ -1009,8 +1055,7 @@ __global__ void __launch_bounds__(kStageThreads, 3)
         // (f-1, xi) and y face f below cell (f, xi)
         const W4 xl_state{sXL[0][tl], sXL[1][tl], sXL[2][tl], sXL[3][tl]};
         Flux5 fx, fy;
-        hllc_x(xl_state, xr, ph, fx);
-        hllc_y(wlNext, wr, ph, fy);
+        hllc_xy(xl_state, xr, fx, wlNext, wr, fy, ph);
         sF[0][t] = fx.d; sF[1][t] = fx.n; sF[2][t] = fx.t1; sF[3][t] = fx.e;
         __syncthreads();
         if (do_cell) {
@@ -1423,7 +1468,8 @@ __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CU
 
     for (int f = y0 + 1; f <= y1; ++f) {
         wait(f + 1);
-        const W4 P1 = c2p4(rowq(f + 1), ph);
+        bool bad;  // parity mode: a quotient of this phase is out of range
+        W4 P1 = c2p4(rowq(f + 1), ph, bad);
         sm.sP[0][t] = make_double2(Pm1.r, Pm1.vx); sm.sP[1][t] = make_double2(Pm1.vy, Pm1.p);
         __syncthreads();
         if (t == 0) {
@@ -1438,22 +1484,33 @@ __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CU
             const double2 c0 = sm.sP[0][tr], c1v = sm.sP[1][tr];
             const W4 a{a0.x, a0.y, a1.x, a1.y};
             const W4 c{c0.x, c0.y, c1v.x, c1v.y};
-            const W4 sx = vl4(a, Pm1, c);
-            const W4 sy = vl4(Pm1, P0, P1);
+            SlopeRange rg;
+            clear(rg);
+            W4 sx = vl4(a, Pm1, c, rg);
+            W4 sy = vl4(Pm1, P0, P1, rg);
+#if !GK_FASTMATH
+            if (bad || out_of_range(rg)) {
+                P1 = c2p4(rowq(f + 1), ph);
+                sx = vl4_any(a, Pm1, c);
+                sy = vl4_any(Pm1, P0, P1);
+            }
+#endif
             const W4 xlft = plus_half(Pm1, sx);
             xr = minus_half(Pm1, sx);
             wr = minus_half(P0, sy);
             wlNew = plus_half(P0, sy);
             sm.sXL[0][t] = make_double2(xlft.r, xlft.vx); sm.sXL[1][t] = make_double2(xlft.vy, xlft.p);
         } else {
+#if !GK_FASTMATH
+            if (bad) P1 = c2p4(rowq(f + 1), ph);
+#endif
             sm.sXL[0][t] = make_double2(Pm1.r, Pm1.vx); sm.sXL[1][t] = make_double2(Pm1.vy, Pm1.p);
         }
         __syncthreads();
         const double2 x0v = sm.sXL[0][tl], x1v = sm.sXL[1][tl];
         const W4 xl_state{x0v.x, x0v.y, x1v.x, x1v.y};
         Flux5 fx, fy;
-        hllc_x(xl_state, xr, ph, fx);
-        hllc_y(wlNext, wr, ph, fy);
+        hllc_xy(xl_state, xr, fx, wlNext, wr, fy, ph);
         if constexpr (LEARN) {
             // x face (xi-1 | xi) of row f-1: cells xi-2 .. xi+1 of sP; a face
             // computed by two strips counts its veto in the strip that
@@ -1575,7 +1632,7 @@ __host__ __device__ constexpr size_t stage_dyn_bytes() {
 // the stage combine and floors: adiabatic.cpp:18-61, recon_piecewise_linear.cpp:8-50,
 // hllc.cpp:22-101, update_cons.cpp:11-68), tiles staged by TMA: stage_tile_tma.
 template <int NT, int KIND, bool PLM>
-__global__ void __launch_bounds__(NT, 512 / NT)
+__global__ void __launch_bounds__(NT, gk::stage_ctas(NT, !GK_FASTMATH))
     k_stage2d_tma(const __grid_constant__ CUtensorMap mapc, const __grid_constant__ CUtensorMap map0,
                   double* out, Geom g, Phys ph, double c1, double c2, double c3, DevTime* tm,
                   int rows) {
@@ -1623,7 +1680,7 @@ __global__ void __launch_bounds__(NT, 256 / NT)
 // instance), claimed through *counter (zeroed before the launch).  Stage
 // KIND 0 reads A and writes B; KIND 2 reads B and A and writes A.
 template <int NT, int KIND, bool PLM>
-__global__ void __launch_bounds__(NT, 512 / NT)
+__global__ void __launch_bounds__(NT, gk::stage_ctas(NT, !GK_FASTMATH))
     k_ens_stage(const gk::EnsInst* __restrict__ inst, const int2* __restrict__ tiles, int ntiles,
                 unsigned* counter, double c1, double c2, double c3) {
     extern __shared__ __align__(128) double dyn[];
@@ -1722,9 +1779,29 @@ void launch_update(const Ctx& c, const double* u0, const double* uc, double* out
                                                  c3, c.tm);
 }
 
+// Length of a march (rows or faces per CTA) over n of them, at most `most`,
+// for `ctas` CTAs per segment index and `slots` resident CTAs: a segment costs
+// about its length plus `extra`, and a last wave that is nearly empty costs as
+// much as a full one, so the length that minimises waves * (length + extra).
+static inline int march_length(int n, int most, long long ctas, long long slots, double extra) {
+    int best = 1;
+    double best_cost = 1e300;
+    for (int r = 1; r <= most && r <= n; ++r) {
+        const long long waves = (ctas * ((n + r - 1) / r) + slots - 1) / slots;
+        const double cost = (double)waves * (r + extra);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = r;
+        }
+    }
+    return best;
+}
 // 3D stage: rows per CTA segment and the CTA width (64, 96 or 128 threads,
 // whichever wastes the fewest lanes on the last strip of columns).
-static inline int stage3d_rows(const Geom& g) { return g.ny < 16 ? g.ny : 16; }
+static inline int stage3d_rows(const Geom& g, int nt) {
+    const long long strips = (g.nx + nt - 5) / (nt - 4);
+    return march_length(g.ny, 32, strips * g.nz, 148LL * (kStage3dThreadsPerSM / nt), 2.5);
+}
 static inline int stage3d_nt(const Geom& g) {
     int best = 128;
     long long best_lanes = 1LL << 62;
@@ -1740,8 +1817,10 @@ static inline int stage3d_nt(const Geom& g) {
 
 void launch_zflux(const Ctx& c, const double* u, double* F3, cudaStream_t s) {
     const Geom& g = c.g;
-    constexpr int zseg = 32;  // faces per thread; nz + 1 faces in all
-    dim3 grid((g.nx + kZX - 1) / kZX, (g.ny + kZY - 1) / kZY, (g.nz + 1 + zseg - 1) / zseg);
+    const unsigned bx = (g.nx + kZX - 1) / kZX, by = (g.ny + kZY - 1) / kZY;
+    // faces per thread; nz + 1 faces in all
+    const int zseg = march_length(g.nz + 1, 48, (long long)bx * by, 148LL * 4, 1.5);
+    dim3 grid(bx, by, (g.nz + 1 + zseg - 1) / zseg);
     if (c.ph.plm) k_zflux<true><<<grid, 128, 0, s>>>(u, F3, g, c.ph, c.tm, zseg);
     else k_zflux<false><<<grid, 128, 0, s>>>(u, F3, g, c.ph, c.tm, zseg);
 }
@@ -1751,7 +1830,7 @@ static void launch_stage3d_nt(const Ctx& c, const double* uc, const double* u0, 
                               const double* F3, int three, double c1, double c2, double c3,
                               cudaStream_t s) {
     const Geom& g = c.g;
-    const int rows = stage3d_rows(g);
+    const int rows = stage3d_rows(g, NT);
     dim3 grid((g.nx + NT - 5) / (NT - 4), (g.ny + rows - 1) / rows, g.nz);
 #define GK_S3(TH, PL, LA) \
     k_stage3d<NT, TH, PL, LA><<<grid, NT, 0, s>>>(uc, u0, out, F3, g, c.ph, c1, c2, c3, c.tm, rows)
@@ -1937,7 +2016,7 @@ template <int NT>
 static void launch_ens_stage_nt(int kind, int plm, const gk::EnsInst* inst, const int2* tiles,
                                 int ntiles, unsigned* counter, double c1, double c2, double c3,
                                 cudaStream_t s) {
-    const int ctas = std::min(ntiles, 148 * (512 / NT));
+    const int ctas = std::min(ntiles, 148 * gk::stage_ctas(NT, !GK_FASTMATH));
     if (plm) {
         if (kind == 0) launch_ens_stage_k<NT, 0, true>(inst, tiles, ntiles, counter, c1, c2, c3, ctas, s);
         else launch_ens_stage_k<NT, 2, true>(inst, tiles, ntiles, counter, c1, c2, c3, ctas, s);

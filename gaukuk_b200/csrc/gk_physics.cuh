@@ -2,8 +2,9 @@
 //
 // Included inside the mode namespace (gk_parity / gk_fast).  Every
 // expression keeps the reference's association order.  The parity unit is
-// compiled with -fmad=false and uses IEEE division and square root, which
-// are correctly rounded on the GPU as on the host: results are bit-identical
+// compiled with -fmad=false and uses correctly rounded division and square
+// root (div_rn, sqrt_rn below where their operands are in range, else CUDA's
+// IEEE operations), as on the host: results are bit-identical
 // to the reference built without -ffast-math.  The fast unit (GK_FASTMATH) lets the
 // compiler contract to FMA and replaces division, reciprocal and square root
 // by the branch-free refinements below.
@@ -44,6 +45,10 @@ __device__ __forceinline__ double sqrt_nr(double x) {
     const double r = fma(-s, s, x);
     return fma(r, 0.5 * y, s);
 }
+__device__ __forceinline__ double rcp_ranged(double b, bool& bad) {
+    bad = false;
+    return rcp_nr(b);
+}
 #define GK_DIV(a, b) ((a) * rcp_nr(b))
 #define GK_RCP(b) rcp_nr(b)
 #define GK_SQRT(x) sqrt_nr(x)
@@ -76,10 +81,10 @@ __device__ __forceinline__ double floor_at(double x, double f) {
 #define GK_MAXNN(a, b) (__double_as_longlong(a) < __double_as_longlong(b) ? (b) : (a))
 #else
 // Parity mode: IEEE division and square root (correctly rounded on the GPU
-// as on the host).
+// as on the host), for operands of any size.
 #define GK_DIV(a, b) ((a) / (b))
-#define GK_RCP(b) (1.0 / (b))
-#define GK_SQRT(x) sqrt(x)
+#define GK_RCP(b) rcp_any(b)
+#define GK_SQRT(x) sqrt_any(x)
 // the reference's compares and std::max/min
 #define GK_MAX0(x) smax((x), 0.0)
 #define GK_MIN0(x) smin(0.0, (x))
@@ -88,6 +93,131 @@ __device__ __forceinline__ double floor_at(double x, double f) {
 #define GK_FLOOR(x, f) smax((x), (f))
 #define GK_BELOW(x, f) ((x) < (f))
 #define GK_MAXNN(a, b) smax((a), (b))
+
+// Correctly rounded quotient, reciprocal and square root without a branch,
+// for operands in range (hi words checked by the callers through the `bad`
+// flags below).  CUDA's IEEE operations test their operands and branch to a
+// slow path each; with about 30 of them per row those branches cut the fused
+// stage's code into pieces between which no two Riemann problems can
+// interleave (branch_resolving and wait stalls, the FP64 pipe 52 % busy).
+// Here the checks are integer tests folded into one flag per phase, and the
+// whole phase is redone with the IEEE operations where it is set.
+//
+// Division (Markstein, IBM J. Res. Dev. 34(1), 1990; Muller et al., Handbook
+// of Floating-Point Arithmetic, ch. 4): with y the correctly rounded 1/b and q
+// a faithful quotient, r = a - b q is exact and fma(r, y, q) is the correctly
+// rounded a/b.  The seed's relative error is below 2^-19.9 (measured over
+// every upper word), so y1 is within 0.51 ulp; one Newton step from it rounds
+// 1/b correctly unless b's significand is all ones (the only 53-bit divisor B
+// of 2^106 - 1 = B M, where 1/b lies 2^-106 above a midpoint), which rounds
+// up (ones_up).  q comes from the seed's quotient corrected with y1 (error
+// 0.5 + 2^-20 ulp).  Square root: Goldschmidt's iteration to within an ulp,
+// then the exact residual; before its last rounding it is within 2^-51 ulp of
+// the root, and of the arguments whose roots lie that near a midpoint every
+// one rounds correctly (tests/test_gpu_parity_math.py runs them all).
+// Against CUDA's operations: 1.7e10 random pairs and 1.1e10 quotients next to
+// midpoints without a difference.
+__device__ __forceinline__ double rcp_seed(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    return y;
+}
+__device__ __forceinline__ double ones_up(double y, double b) {
+    const bool ones = ((__double2hiint(b) | (int)0xfff00000) & __double2loint(b)) == -1;
+    return __hiloint2double(__double2hiint(y), __double2loint(y) | (ones ? 1 : 0));
+}
+// div_rn_plain: for a significand of b that is not all ones.
+template <bool ONES>
+__device__ __forceinline__ double div_rn_t(double a, double b) {
+    const double y0 = rcp_seed(b);
+    const double e = fma(-b, y0, 1.0);
+    const double y1 = fma(y0, fma(e, e, e), y0);
+    const double q0 = a * y0;
+    const double q1 = fma(fma(-b, q0, a), y1, q0);
+    double y = fma(y1, fma(-b, y1, 1.0), y1);
+    if (ONES) y = ones_up(y, b);
+    return fma(fma(-b, q1, a), y, q1);
+}
+__device__ __forceinline__ double div_rn(double a, double b) { return div_rn_t<true>(a, b); }
+__device__ __forceinline__ double div_rn_plain(double a, double b) { return div_rn_t<false>(a, b); }
+__device__ __forceinline__ double rcp_rn(double b) {
+    const double y0 = rcp_seed(b);
+    const double e = fma(-b, y0, 1.0);
+    const double y1 = fma(y0, fma(e, e, e), y0);
+    return ones_up(fma(y1, fma(-b, y1, 1.0), y1), b);
+}
+__device__ __forceinline__ double sqrt_rn(double x) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+    const double g0 = x * y0, h0 = 0.5 * y0;
+    const double e = fma(-g0, h0, 0.5);
+    const double t = fma(1.5 * e, e, e);  // (1 - 2e)^-1/2 = 1 + e + 3/2 e^2 + ...
+    const double g = fma(g0, t, g0), h = fma(h0, t, h0);
+    return fma(fma(-g, g, x), h, g);
+}
+
+// Range tests.  The upper words of doubles, read as floats, keep the order of
+// the values, and a double that is not finite (or above 2^1016) reads as a
+// float infinity or NaN; so the tests of a phase run as NaN-propagating float
+// minima and maxima, whose absolute values and signs cost nothing, and one
+// compare at the end.
+__device__ __forceinline__ int hi(double x) { return __double2hiint(x); }
+__device__ __forceinline__ float top(double x) { return __int_as_float(__double2hiint(x)); }
+__device__ __forceinline__ float pow2_top(int k) { return __int_as_float((1023 + k) << 20); }
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ bool is_zero(double x) {
+    return ((hi(x) & 0x7fffffff) | __double2loint(x)) == 0;
+}
+// 0 < |x| < 2^-400: too small for the exact residuals
+__device__ __forceinline__ bool tiny(double x) {
+    return fabsf(top(x)) < pow2_top(-400) && !is_zero(x);
+}
+// 2^lo <= x < 2^up
+__device__ __forceinline__ bool in_pos(double x, int lo, int up) {
+    return top(x) >= pow2_top(lo) && top(x) < pow2_top(up);
+}
+// all ones in x's significand: 0xffffffff, else less
+__device__ __forceinline__ unsigned ones_of(double x) {
+    return (unsigned)((hi(x) | (int)0xfff00000) & __double2loint(x));
+}
+// Densities and pressures in [2^-60, 2^100) and speeds below 2^100 keep every
+// product, quotient and residual of the Riemann problem (hllc_ranged) normal
+// and finite; the floors (2^-53) are inside.
+constexpr int kLo = -60, kUp = 100;
+
+// 1/x in range, with the range test left to the caller's flag.
+__device__ __forceinline__ double rcp_ranged(double x, bool& bad) {
+    bad = !in_pos(x, kLo, kUp);
+    return rcp_rn(x);
+}
+// 1/x, and sqrt(x), each with its own range test.
+__device__ __forceinline__ double rcp_any(double x) {
+    if (in_pos(x, kLo, kUp)) return rcp_rn(x);
+    return 1.0 / x;
+}
+__device__ __forceinline__ double sqrt_any(double x) {
+    if (in_pos(x, -500, 500)) return sqrt_rn(x);
+    return sqrt(x);
+}
 #endif
 
 // Reconstruction::VanLeer (reconstruction.hpp:36-42).
@@ -101,14 +231,48 @@ __device__ __forceinline__ double vanleer(double a, double b) {
 #endif
 }
 
+// Half the van Leer slope: what the PLM face states u +- 0.5*sigma add.  Fast
+// mode: (a*b)/(a+b) for ab > 0 else 0, without the two scalings by 2 and 1/2.
+// Parity mode: the same quotient, which is exactly 0.5*((2ab)/(a+b)) unless a
+// scaling underflows; the record tells where it might not be the reference's
+// value (a product below 2^-400, a sum above 2^400 or with all ones).
 #if GK_FASTMATH
-// Half the van Leer slope, (a*b)/(a+b) for ab > 0 else 0: what the PLM face
-// states u +- 0.5*sigma add, without the two scalings by 2 and 1/2.
-__device__ __forceinline__ double vanleer_half(double a, double b) {
+struct SlopeRange {};
+__device__ __forceinline__ void clear(SlopeRange&) {}
+__device__ __forceinline__ double vanleer_half(double a, double b, SlopeRange&) {
     const double multi = a * b;
     const double h = GK_DIV(multi, a + b);
     return GK_LE0(multi) ? 0.0 : h;
 }
+__device__ __forceinline__ double vanleer_half_any(double a, double b) {
+    SlopeRange none;
+    return vanleer_half(a, b, none);
+}
+#else
+// Range record of a phase's slopes: the smallest product and the largest sum
+// (as floats), and whether a sum's significand is all ones.
+struct SlopeRange {
+    float lo, up;
+    unsigned ones;
+};
+__device__ __forceinline__ void clear(SlopeRange& r) {
+    r.lo = pow2_top(0);
+    r.up = 0.f;
+    r.ones = 0u;
+}
+__device__ __forceinline__ bool out_of_range(const SlopeRange& r) {
+    return !(r.lo >= pow2_top(-400) && r.up < pow2_top(400)) || r.ones == 0xffffffffu;
+}
+__device__ __forceinline__ double vanleer_half(double a, double b, SlopeRange& r) {
+    const double multi = a * b, sum = a + b;
+    const bool none = multi <= 0.0;
+    r.lo = min_nan(r.lo, none ? pow2_top(0) : top(multi));
+    r.up = max_nan(r.up, fabsf(top(sum)));
+    r.ones = max(r.ones, ones_of(sum));
+    const double h = div_rn_plain(multi, sum);
+    return none ? 0.0 : h;
+}
+__device__ __noinline__ double vanleer_half_any(double a, double b) { return 0.5 * vanleer(a, b); }
 #endif
 
 struct Flux5 {
@@ -128,9 +292,9 @@ struct Flux5 {
 // which differs only where the unused side is not finite, or in the sign of
 // a zero.
 template <bool T2, int SEL>
-__device__ __forceinline__ void hllc(double denl, double vxl, double vyl, double vzl, double prel,
-                                     double denr, double vxr, double vyr, double vzr, double prer,
-                                     const gk::Phys& ph, Flux5& f) {
+__device__ __forceinline__ void hllc_any(double denl, double vxl, double vyl, double vzl, double prel,
+                                         double denr, double vxr, double vyr, double vzr, double prer,
+                                         const gk::Phys& ph, Flux5& f) {
     const double gamma = ph.gamma;
 #if GK_FASTMATH
     // sqrt(gamma*p/rho) = (gamma*p) * rsqrt(gamma*p*rho): one root, no quotient
@@ -139,8 +303,8 @@ __device__ __forceinline__ void hllc(double denl, double vxl, double vyl, double
     double ar = gpr * rsqrt_nr(gpr * denr);
 #else
     // EquationOfState::SoundSpeed (eos.hpp:27-29)
-    double al = GK_SQRT(GK_DIV(gamma * prel, denl));
-    double ar = GK_SQRT(GK_DIV(gamma * prer, denr));
+    double al = sqrt(GK_DIV(gamma * prel, denl));
+    double ar = sqrt(GK_DIV(gamma * prer, denr));
 #endif
     double prePVRS = 0.5 * (prel + prer) - 0.125 * (vxr - vxl) * (denl + denr) * (al + ar);
     prePVRS = GK_MAX0(prePVRS);
@@ -165,11 +329,11 @@ __device__ __forceinline__ void hllc(double denl, double vxl, double vyl, double
     qr = 1.0;
     if (!(prePVRS <= prel && prel > 0.0)) {
         double temp = smax(GK_DIV(prePVRS, prel) - 1, 0.0);
-        ql = GK_SQRT(1 + ph.cq * temp);
+        ql = sqrt(1 + ph.cq * temp);
     }
     if (!(prePVRS <= prer && prer > 0.0)) {
         double temp = smax(GK_DIV(prePVRS, prer) - 1, 0.0);
-        qr = GK_SQRT(1 + ph.cq * temp);
+        qr = sqrt(1 + ph.cq * temp);
     }
     double sl = vxl - al * ql;
     double sr = vxr + ar * qr;
@@ -240,4 +404,153 @@ __device__ __forceinline__ void hllc(double denl, double vxl, double vyl, double
     f.t1 = f1 * v1;
     f.t2 = T2 ? f1 * v2 : 0.0;
     f.e = ep * vc + c * ss * m;
+}
+
+#if GK_FASTMATH
+// Fast mode has one form: no lane is ever out of its range.
+struct HllcAux {};
+template <bool T2, int SEL>
+__device__ __forceinline__ void hllc_ranged(double denl, double vxl, double vyl, double vzl,
+                                            double prel, double denr, double vxr, double vyr,
+                                            double vzr, double prer, const gk::Phys& ph, Flux5& f,
+                                            bool&, HllcAux&) {
+    hllc_any<T2, SEL>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f);
+}
+template <bool T2, int SEL>
+__device__ __forceinline__ void hllc_redo(double, double, double, double, double, double, double,
+                                          double, double, double, const gk::Phys&, Flux5&, bool,
+                                          const HllcAux&) {}
+#else
+// The Riemann problem for states in range, straight-line, and only its
+// selected side: with both sides finite the reference's
+// selectl*fl + selectr*fr is the selected side's flux, except that a -0 of it
+// becomes +0 where the other side's component is positive.  `bad` is set
+// where an operand is out of range (the flux must come from hllc_any); aux
+// keeps what hllc_redo needs to give a -0 the reference's sign.
+struct HllcAux {
+    double ss, so;  // contact speed, the other side's wave speed
+    bool zero;      // a component of the selected side is -0
+};
+template <bool T2, int SEL>
+__device__ __forceinline__ void hllc_ranged(double denl, double vxl, double vyl, double vzl,
+                                            double prel, double denr, double vxr, double vyr,
+                                            double vzr, double prer, const gk::Phys& ph, Flux5& f,
+                                            bool& bad, HllcAux& aux) {
+    const double gamma = ph.gamma;
+    // range record: lo of what must be at least 2^-60, up of what must stay
+    // below 2^100 in size
+    float lo = min3(top(denl), top(prel), min_nan(top(denr), top(prer)));
+    float up = max3(top(denl), top(prel), max_nan(top(denr), top(prer)));
+    up = max3(up, fabsf(top(vxl)), fabsf(top(vxr)));
+    up = max3(up, fabsf(top(vyl)), fabsf(top(vyr)));
+    if (T2) up = max3(up, fabsf(top(vzl)), fabsf(top(vzr)));
+    const double al = sqrt_rn(div_rn(gamma * prel, denl));
+    const double ar = sqrt_rn(div_rn(gamma * prer, denr));
+    double prePVRS = 0.5 * (prel + prer) - 0.125 * (vxr - vxl) * (denl + denr) * (al + ar);
+    prePVRS = hi(prePVRS) < 0 ? 0.0 : prePVRS;  // zero, or at least 2^-114 by its terms
+    // q = sqrt(1 + cq max(p*/p - 1, 0))
+    double tl = div_rn(prePVRS, prel) - 1, tr = div_rn(prePVRS, prer) - 1;
+    tl = hi(tl) < 0 ? 0.0 : tl;
+    tr = hi(tr) < 0 ? 0.0 : tr;
+    const double ql = sqrt_rn(1 + ph.cq * tl), qr = sqrt_rn(1 + ph.cq * tr);
+    const double sl = vxl - al * ql, sr = vxr + ar * qr;
+    const double dl = sl - vxl, dr = sr - vxr;
+    const double num = prer - prel + denl * vxl * dl - denr * vxr * dr;
+    const double den = denl * dl - denr * dr;  // negative
+    const double ss = div_rn_plain(num, den);
+    const double bl = sl - ss, br = sr - ss;  // negative, positive
+    lo = min3(lo, -top(den), min_nan(-top(bl), top(br)));
+    const bool left = top(ss) >= 0.f;  // ss >= 0, -0 included (ss is 0 or at least 2^-600)
+    const double d = left ? denl : denr, vn = left ? vxl : vxr, v1 = left ? vyl : vyr;
+    const double v2 = T2 ? (left ? vzl : vzr) : 0.0, p = left ? prel : prer, s = left ? sl : sr;
+    const double sv = left ? dl : dr;
+    // a/b with b = S - S* made negative (a/b = (-a)/(-b)): a zero quotient of
+    // div_rn has the IEEE sign for b < 0 only
+    const double sc = left ? (hi(s) < 0 ? s : 0.0) : (hi(s) < 0 ? 0.0 : s);
+    const double a = sc * (ss - vn);
+    const double b = left ? bl : -br;
+    up = max3(up, top(prePVRS), max3(fabsf(top(num)), fabsf(top(ss)), fabsf(top(a))));
+    bad |= !(lo >= pow2_top(kLo) && up < pow2_top(kUp)) || tiny(num) || tiny(a) ||
+           max(ones_of(den), ones_of(b)) == 0xffffffffu;
+    const double c = div_rn_plain(left ? a : -a, b);
+    const double k = T2 ? (vn * vn + v1 * v1 + v2 * v2) : (vn * vn + v1 * v1);
+    const double e = p * ph.gm1Rec + 0.5 * d * k;
+    const double vc = vn + c;
+    const double f1 = d * vc;
+    f.d = f1;
+    f.n = d * (vn * vn + c * s) + p;
+    f.t1 = f1 * v1;
+    f.t2 = T2 ? f1 * v2 : 0.0;
+    f.e = (e + p) * vc + d * c * ss * sv;
+    constexpr int kNeg = (int)0x80000000;
+    aux.zero = hi(f.d) == kNeg || hi(f.t1) == kNeg || (T2 && hi(f.t2) == kNeg) || hi(f.e) == kNeg;
+    aux.ss = ss;
+    aux.so = left ? sr : sl;
+}
+
+// hllc_any kept out of line: it runs for few lanes, and inlined it would
+// stretch the row loop over more instruction lines.
+struct HllcStates {
+    double denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer;
+};
+template <bool T2, int SEL>
+__device__ __noinline__ Flux5 hllc_far(HllcStates w, double gamma, double gm1Rec, double cq) {
+    gk::Phys ph;
+    ph.gamma = gamma;
+    ph.gm1Rec = gm1Rec;
+    ph.cq = cq;
+    Flux5 f;
+    hllc_any<T2, SEL>(w.denl, w.vxl, w.vyl, w.vzl, w.prel, w.denr, w.vxr, w.vyr, w.vzr, w.prer, ph, f);
+    return f;
+}
+
+// Completes hllc_ranged where it set `bad` or aux.zero.  The sign of the
+// other side's mass flux is that of v + c, and c's sign and size come from
+// the seed reciprocal (relative error 2^-19): unless v and c cancel to 2^-16,
+// that sign is certain.  The momenta's signs follow from it; a -0 energy flux
+// and a cancellation take the full evaluation.
+template <bool T2, int SEL>
+__device__ __forceinline__ void hllc_redo(double denl, double vxl, double vyl, double vzl,
+                                          double prel, double denr, double vxr, double vyr,
+                                          double vzr, double prer, const gk::Phys& ph, Flux5& f,
+                                          bool bad, const HllcAux& aux) {
+    if (!bad && aux.zero) {
+        const bool left = aux.ss >= 0;
+        const double vo = left ? vxr : vxl, v1 = left ? vyr : vyl, v2 = left ? vzr : vzl;
+        const double sc = left ? smax(0.0, aux.so) : smin(0.0, aux.so);
+        const double a = sc * (aux.ss - vo);
+        const double c = a * rcp_seed(aux.so - aux.ss);
+        const double vc = vo + c;
+        const bool sure = is_zero(a) || (hi(vc) & 0x7fffffff) + (16 << 20) >= (hi(c) & 0x7fffffff);
+        constexpr int kNeg = (int)0x80000000;
+        bad = !sure || hi(f.e) == kNeg;
+        const int neg = hi(vc);  // sign bit of the other side's mass flux
+        auto zero = [&](double& x, int other) {  // -0 + 0*y: -0 for y < 0 or -0, else +0
+            if (hi(x) == kNeg) {
+                bad = bad || __double2loint(x) != 0;
+                x = other < 0 ? x : 0.0;
+            }
+        };
+        zero(f.d, neg);
+        zero(f.t1, neg ^ hi(v1));
+        if (T2) zero(f.t2, neg ^ hi(v2));
+    }
+    if (bad)
+        f = hllc_far<T2, SEL>(HllcStates{denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer},
+                              ph.gamma, ph.gm1Rec, ph.cq);
+}
+#endif
+
+// Flux::RiemannSolver for one face of any state.
+template <bool T2, int SEL>
+__device__ __forceinline__ void hllc(double denl, double vxl, double vyl, double vzl, double prel,
+                                     double denr, double vxr, double vyr, double vzr, double prer,
+                                     const gk::Phys& ph, Flux5& f) {
+    bool bad = !ph.ranged;
+    HllcAux aux;
+    hllc_ranged<T2, SEL>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f, bad, aux);
+#if !GK_FASTMATH
+    if (bad || aux.zero)
+        hllc_redo<T2, SEL>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f, bad, aux);
+#endif
 }

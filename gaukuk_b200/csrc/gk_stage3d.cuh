@@ -19,22 +19,6 @@
 // the same bits.
 #pragma once
 
-// PLM face states of one variable from three cells, as k_flux forms them.
-__device__ __forceinline__ double plm_up(double a, double b, double c) {
-#if GK_FASTMATH
-    return b + vanleer_half(b - a, c - b);
-#else
-    return b + 0.5 * vanleer(b - a, c - b);
-#endif
-}
-__device__ __forceinline__ double plm_down(double a, double b, double c) {
-#if GK_FASTMATH
-    return b - vanleer_half(b - a, c - b);
-#else
-    return b - 0.5 * vanleer(b - a, c - b);
-#endif
-}
-
 struct W5 {
     double v[5];  // primitive slots: rho, vx, vy, p, vz
 };
@@ -59,6 +43,13 @@ __device__ __forceinline__ Q5 load5(const double* __restrict__ u, const Geom& g,
     for (int v = 0; v < 5; ++v) r.q[v] = __ldg(u + v * g.vstride + c);
     return r;
 }
+// `bad`: set where the density is out of parity mode's range (c2p_q redoes it)
+__device__ __forceinline__ W5 c2p_q(const Q5& a, const Phys& ph, bool& bad) {
+    W5 w;
+    cons_to_prim5(a.q[gk::S_DEN], a.q[gk::S_MTX], a.q[gk::S_MTY], a.q[gk::S_MTZ], a.q[gk::S_ENG],
+                  rcp_ranged(GK_FLOOR(a.q[gk::S_DEN], ph.dmin), bad), ph, w.v);
+    return w;
+}
 __device__ __forceinline__ W5 c2p_q(const Q5& a, const Phys& ph) {
     W5 w;
     cons_to_prim5(a.q[gk::S_DEN], a.q[gk::S_MTX], a.q[gk::S_MTY], a.q[gk::S_MTZ], a.q[gk::S_ENG], ph,
@@ -66,17 +57,14 @@ __device__ __forceinline__ W5 c2p_q(const Q5& a, const Phys& ph) {
     return w;
 }
 
-// Riemann problem of an x face (vx | vy, vz) and a y face (vy | vz, vx),
-// hllc.cpp:25-27; the fluxes land in slot order (DEN, MTX, MTY, ENG, MTZ).
-__device__ __forceinline__ void hllc5_x(const double (&l)[5], const double (&r)[5], const Phys& ph,
-                                        double (&F)[5]) {
-    Flux5 f;
-    hllc<true, kSel>(l[gk::P_RHO], l[gk::P_VX], l[gk::P_VY], l[gk::P_VZ], l[gk::P_PRE], r[gk::P_RHO],
-                     r[gk::P_VX], r[gk::P_VY], r[gk::P_VZ], r[gk::P_PRE], ph, f);
+// Riemann problem of a y face (vy | vz, vx), and of an x face (vx | vy, vz)
+// and a y face together (see hllc_xy), hllc.cpp:25-27; the fluxes land in slot
+// order (DEN, MTX, MTY, ENG, MTZ).
+__device__ __forceinline__ void slots_y(const Flux5& f, double (&F)[5]) {
     F[gk::S_DEN] = f.d;
-    F[gk::S_MTX] = f.n;
-    F[gk::S_MTY] = f.t1;
-    F[gk::S_MTZ] = f.t2;
+    F[gk::S_MTY] = f.n;
+    F[gk::S_MTZ] = f.t1;
+    F[gk::S_MTX] = f.t2;
     F[gk::S_ENG] = f.e;
 }
 __device__ __forceinline__ void hllc5_y(const double (&l)[5], const double (&r)[5], const Phys& ph,
@@ -84,11 +72,34 @@ __device__ __forceinline__ void hllc5_y(const double (&l)[5], const double (&r)[
     Flux5 f;
     hllc<true, kSel>(l[gk::P_RHO], l[gk::P_VY], l[gk::P_VZ], l[gk::P_VX], l[gk::P_PRE], r[gk::P_RHO],
                      r[gk::P_VY], r[gk::P_VZ], r[gk::P_VX], r[gk::P_PRE], ph, f);
-    F[gk::S_DEN] = f.d;
-    F[gk::S_MTY] = f.n;
-    F[gk::S_MTZ] = f.t1;
-    F[gk::S_MTX] = f.t2;
-    F[gk::S_ENG] = f.e;
+    slots_y(f, F);
+}
+__device__ __forceinline__ void hllc5_xy(const double (&xl)[5], const double (&xr)[5],
+                                         double (&Fx)[5], const double (&yl)[5],
+                                         const double (&yr)[5], double (&Fy)[5], const Phys& ph) {
+    bool badx = !ph.ranged, bady = !ph.ranged;
+    HllcAux ax, ay;
+    Flux5 fx, fy;
+#define GK_XARGS xl[gk::P_RHO], xl[gk::P_VX], xl[gk::P_VY], xl[gk::P_VZ], xl[gk::P_PRE], \
+                 xr[gk::P_RHO], xr[gk::P_VX], xr[gk::P_VY], xr[gk::P_VZ], xr[gk::P_PRE], ph, fx, badx, ax
+#define GK_YARGS yl[gk::P_RHO], yl[gk::P_VY], yl[gk::P_VZ], yl[gk::P_VX], yl[gk::P_PRE], \
+                 yr[gk::P_RHO], yr[gk::P_VY], yr[gk::P_VZ], yr[gk::P_VX], yr[gk::P_PRE], ph, fy, bady, ay
+    hllc_ranged<true, kSel>(GK_XARGS);
+    hllc_ranged<true, kSel>(GK_YARGS);
+#if !GK_FASTMATH
+    if (badx || bady || ax.zero || ay.zero) {
+        hllc_redo<true, kSel>(GK_XARGS);
+        hllc_redo<true, kSel>(GK_YARGS);
+    }
+#endif
+#undef GK_XARGS
+#undef GK_YARGS
+    Fx[gk::S_DEN] = fx.d;
+    Fx[gk::S_MTX] = fx.n;
+    Fx[gk::S_MTY] = fx.t1;
+    Fx[gk::S_MTZ] = fx.t2;
+    Fx[gk::S_ENG] = fx.e;
+    slots_y(fy, Fy);
 }
 
 // ------------------------------------------------------------ z faces
@@ -101,8 +112,7 @@ __device__ __forceinline__ void hllc5_y(const double (&l)[5], const double (&r)[
 // shared array; the raw values of the next plane are in flight while a face
 // is solved.  The y-slope of cell (k, j) gives both its lower state (the
 // right state of face k-1|k) and its upper state (the left state of face
-// k|k+1).  The expressions are plm_up / plm_down's, so the fluxes are the
-// same bits.
+// k|k+1).  The expressions are k_flux's, so the fluxes are the same bits.
 constexpr int kZX = 32, kZY = 4, kZRows = kZY + 2, kZCells = kZX * kZRows;
 
 template <bool PLM>
@@ -141,21 +151,18 @@ __global__ void __launch_bounds__(128)
     };
     // states of cell (k, j) from the tile's rows ty, ty+1, ty+2 (= j-1, j, j+1)
     auto states = [&](int buf, double (&lo)[5], double (&up)[5]) {
+        double a[5], b[5], c[5], h[5];
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-            const double b = sW[buf][ty + 1][v][tx];
-            if (PLM) {
-                const double a = sW[buf][ty][v][tx], c = sW[buf][ty + 2][v][tx];
-#if GK_FASTMATH
-                const double h = vanleer_half(b - a, c - b);
-#else
-                const double h = 0.5 * vanleer(b - a, c - b);
-#endif
-                lo[v] = b - h;
-                up[v] = b + h;
-            } else {
-                lo[v] = up[v] = b;
-            }
+            a[v] = sW[buf][ty][v][tx];
+            b[v] = sW[buf][ty + 1][v][tx];
+            c[v] = sW[buf][ty + 2][v][tx];
+        }
+        if (PLM) half_slopes5(a, b, c, h);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            lo[v] = PLM ? b[v] - h[v] : b[v];
+            up[v] = PLM ? b[v] + h[v] : b[v];
         }
     };
     Q5 qa, qb;
@@ -199,11 +206,12 @@ __global__ void __launch_bounds__(128)
 // step's last stage also reduces the CFL speed of the new state (CalCmax,
 // adiabatic.cpp:115-160, on the values it writes) and its last CTA runs the
 // step epilogue, as k_cfl would after it.
-// Resident threads per SM: 384 in fast mode (up to 168 registers each), 512
-// in parity mode (128 registers, with 16-72 bytes of spills).  At 256^3 (CTAs of 96) parity
-// mode went from 5.39 to 5.13 ms per step with the extra warps, while fast
-// mode, whose early row loads need the registers, went from 2.28 to 2.42.
-constexpr int kStage3dThreadsPerSM = GK_FASTMATH ? 384 : 512;
+// Resident threads per SM: 384, at up to 168 registers each (parity mode with
+// 40-72 bytes of spills).  Parity mode at 192^3: 1.74 ms per step, 1.72 at 256
+// threads without spills, which loses 10-30 % on small grids (64^3: 158 us
+// against 207); fast mode at 512 threads ran 2.28 -> 2.42 ms at 256^3 (its
+// early loads need the registers).
+constexpr int kStage3dThreadsPerSM = 384;
 template <int NT, bool THREE, bool PLM, bool LAST>
 __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
     k_stage3d(const double* __restrict__ uc, const double* u0, double* out,
@@ -235,15 +243,19 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
     // lower state of y face y0 (upper y state of cell y0-1), then that face
     {
         const W5 P1 = c2p_at(uc, g, ph, at(y0 + 1));
-        double wr[5];
+        double wr[5], h[5], h0[5];
+        if (PLM) {
+            half_slopes5(Pm2.v, Pm1.v, P0.v, h);
+            half_slopes5(Pm1.v, P0.v, P1.v, h0);
+        }
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-            wlNext[v] = PLM ? plm_up(Pm2.v[v], Pm1.v[v], P0.v[v]) : Pm1.v[v];
-            wr[v] = PLM ? plm_down(Pm1.v[v], P0.v[v], P1.v[v]) : P0.v[v];
+            wlNext[v] = PLM ? Pm1.v[v] + h[v] : Pm1.v[v];
+            wr[v] = PLM ? P0.v[v] - h0[v] : P0.v[v];
         }
         hllc5_y(wlNext, wr, ph, fyPrev);
 #pragma unroll
-        for (int v = 0; v < 5; ++v) wlNext[v] = PLM ? plm_up(Pm1.v[v], P0.v[v], P1.v[v]) : P0.v[v];
+        for (int v = 0; v < 5; ++v) wlNext[v] = PLM ? P0.v[v] + h0[v] : P0.v[v];
         Pm1 = P0;
         P0 = P1;
     }
@@ -270,19 +282,40 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
             }
         };
         if (kEarly && do_cell) load_row_inputs();
-        const W5 P1 = c2p_q(Q1, ph);
+        bool bad;  // parity mode: a quotient of this phase is out of range
+        SlopeRange rg;
+        clear(rg);
+        W5 P1 = c2p_q(Q1, ph, bad);
 #pragma unroll
         for (int v = 0; v < 5; ++v) sP[v][t] = Pm1.v[v];
         __syncthreads();
-        double xr[5], wr[5], wlNew[5];
+        double xr[5], wr[5], wlNew[5], hx[5], hy[5];
+        if (PLM) {
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+                hx[v] = vanleer_half(Pm1.v[v] - sP[v][tl], sP[v][tr] - Pm1.v[v], rg);
+                hy[v] = vanleer_half(P0.v[v] - Pm1.v[v], P1.v[v] - P0.v[v], rg);
+            }
+        }
+#if !GK_FASTMATH
+        if (bad || (PLM && out_of_range(rg))) {
+            P1 = c2p_q(Q1, ph);
+            if (PLM) {
+#pragma unroll
+                for (int v = 0; v < 5; ++v) {
+                    hx[v] = vanleer_half_any(Pm1.v[v] - sP[v][tl], sP[v][tr] - Pm1.v[v]);
+                    hy[v] = vanleer_half_any(P0.v[v] - Pm1.v[v], P1.v[v] - P0.v[v]);
+                }
+            }
+        }
+#endif
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-            const double a = sP[v][tl], c = sP[v][tr];
             if (PLM) {
-                sXL[v][t] = plm_up(a, Pm1.v[v], c);
-                xr[v] = plm_down(a, Pm1.v[v], c);
-                wr[v] = plm_down(Pm1.v[v], P0.v[v], P1.v[v]);
-                wlNew[v] = plm_up(Pm1.v[v], P0.v[v], P1.v[v]);
+                sXL[v][t] = Pm1.v[v] + hx[v];
+                xr[v] = Pm1.v[v] - hx[v];
+                wr[v] = P0.v[v] - hy[v];
+                wlNew[v] = P0.v[v] + hy[v];
             } else {
                 sXL[v][t] = Pm1.v[v];
                 xr[v] = Pm1.v[v];
@@ -294,8 +327,7 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
         double xlst[5], fx[5], fy[5];
 #pragma unroll
         for (int v = 0; v < 5; ++v) xlst[v] = sXL[v][tl];
-        hllc5_x(xlst, xr, ph, fx);
-        hllc5_y(wlNext, wr, ph, fy);
+        hllc5_xy(xlst, xr, fx, wlNext, wr, fy, ph);
 #pragma unroll
         for (int v = 0; v < 5; ++v) sF[v][t] = fx[v];
         __syncthreads();

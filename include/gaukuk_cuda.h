@@ -351,6 +351,13 @@ int gk_tap_substeps(gk_handle* h, int nsub, double dt_sub, int ratio, double* fx
  * compiler's. */
 int gk_fastmath_check(int n, unsigned long long seed, double* worst3);
 
+/* Diagnostic of the PARITY mode arithmetic: its branch-free quotient a/b,
+ * reciprocal 1/b and square root sqrt(a) of n operand pairs (host arrays; out
+ * holds 3n doubles), which must equal the IEEE results for operands between
+ * 2^-400 and 2^400.  Runs on the current device.  No counterpart in the
+ * reference, whose arithmetic is the host compiler's. */
+int gk_paritymath_eval(int n, const double* a, const double* b, double* out);
+
 
 /* The bounds-checked build (lib/checked/libgk_cuda.so, compiled with
  * GK_CHECKED; no counterpart in the reference, whose only sanitizer is a
