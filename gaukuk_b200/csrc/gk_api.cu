@@ -125,6 +125,8 @@ struct gk_handle {
     gk::DevTime* htm = nullptr;  // pinned mirror
     double* dlog = nullptr;
     int* dflag = nullptr;
+    double* dstrips = nullptr;  // 2D: a download's ghost strips, gathered (device),
+    double* hstrips = nullptr;  // and their pinned landing place
     int path = 0;  // 0 generic, 1 fused 2D
     bool uploaded = false;
     int upload_step = 0;  // clock step at the last upload
@@ -275,6 +277,10 @@ int build_ctx(gk_handle* h) {
     return GK_OK;
 }
 
+// Doubles of one variable's ghost strips in 2D: two columns of the active rows
+// on each x side, two rows of the active columns on each y side.
+inline size_t strip_doubles(const gk::Geom& g) { return 2 * (size_t)g.ng * (g.nx + g.ny); }
+
 int alloc_state(gk_handle* h) {
     const gk::Geom& g = h->ctx.g;
     size_t bytes = sizeof(double) * 5 * (size_t)g.vstride;
@@ -290,6 +296,11 @@ int alloc_state(gk_handle* h) {
     GK_CUDA(h, cudaMalloc(&h->dlog, sizeof(double) * kLogCap));
     GK_CUDA(h, cudaMalloc(&h->dflag, sizeof(int)));
     GK_CUDA(h, cudaMallocHost(&h->htm, sizeof(gk::DevTime)));
+    if (g.ndim == 2) {
+        const size_t sb = sizeof(double) * 5 * strip_doubles(g);
+        GK_CUDA(h, cudaMalloc(&h->dstrips, sb));
+        GK_CUDA(h, cudaMallocHost(&h->hstrips, sb));
+    }
     gk::DevTime t{};
     t.t = 0; t.dt = 1e10; t.tNext = 0; t.dtUntilOutput = 1e10;  // sim.cpp:45-46
     t.cmax_last = 1e-16;
@@ -651,30 +662,123 @@ int pull_time(gk_handle* h) {
     return GK_OK;
 }
 
-// A reference-layout host state (NVar x lenz x leny x lenx) into a device
-// state buffer (slots DEN, MTX, MTY, ENG, MTZ; stored planes; pitched rows).
-// Stored planes of reference variable n (all five when n < 0).
+// Transfers of a whole state.  The reference layout is dense (NVar x lenz x
+// leny x lenx), the device's rows are pitched and its slots ordered DEN, MTX,
+// MTY, ENG, MTZ.  Where the handle has the generic path's scratch W (1D, 3D,
+// and 2D off the fused path) the state crosses the bus dense, one copy per
+// variable, and a kernel packs or unpacks it: a 3D state took one pitched copy
+// per plane and variable and four per plane for its ghost strips (256^3: 6400
+// copies, 38 ms; now 13 ms, the bus).  On the fused 2D path each variable is
+// one pitched copy and the ghost strips, which come from another buffer, are
+// gathered into one copy and placed by the host.
+__global__ void k_unpack_state(const double* __restrict__ src, double* __restrict__ u, gk::Geom g) {
+    constexpr int slot[5] = {gk::S_DEN, gk::S_MTX, gk::S_MTY, gk::S_MTZ, gk::S_ENG};
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.lenx) return;
+    const int rows = g.nzs * g.leny;  // rows of one variable, planes contiguous
+    for (int r = blockIdx.y; r < 5 * rows; r += gridDim.y) {
+        const int n = r / rows;
+        u[slot[n] * g.vstride + (long long)(r - n * rows) * g.pitch + i] =
+            src[(long long)r * g.lenx + i];
+    }
+}
+
+// The state as the reference leaves it after a step: Sim's integrators end
+// with cons.Swap(consTemp) (rk2.cpp:21, rk3.cpp:27), so the written array
+// carries the ghost fill of the last intermediate stage state.  The ghost
+// strips of active rows, columns and planes therefore come from the stage
+// buffer `donor` once a step has been taken since the upload.
+__device__ __forceinline__ bool from_donor(const gk::Geom& g, int fill_z, int k, int j, int i) {
+    const bool ai = i >= g.ib && i < g.ie, aj = j >= g.jb && j < g.je, ak = k >= g.kb && k < g.ke;
+    if (!ai && g.nx > 1) return aj && ak;
+    if (!aj && g.ny > 1) return ai && ak;
+    if (!ak && g.nz > 1) return ai && aj && ((fill_z >> (k < g.kb ? 0 : 1)) & 1);
+    return false;
+}
+__global__ void k_pack_state(const double* __restrict__ u, const double* __restrict__ donor,
+                             double* __restrict__ dst, gk::Geom g, int fill_z,
+                             const gk::DevTime* __restrict__ tm, int upload_step) {
+    constexpr int slot[5] = {gk::S_DEN, gk::S_MTX, gk::S_MTY, gk::S_MTZ, gk::S_ENG};
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.lenx) return;
+    const bool use = donor && tm->step > upload_step;
+    const int rows = g.nzs * g.leny;
+    for (int r = blockIdx.y; r < 5 * rows; r += gridDim.y) {
+        const int n = r / rows, q = r - n * rows;
+        const bool other = use && from_donor(g, fill_z, g.kofs + q / g.leny, q % g.leny, i);
+        dst[(long long)r * g.lenx + i] =
+            (other ? donor : u)[slot[n] * g.vstride + (long long)q * g.pitch + i];
+    }
+}
+// 2D: per slot the x strips [side][row][2], then the y strips [side][2][column].
+__global__ void k_gather_strips(const double* __restrict__ u, const double* __restrict__ donor,
+                                double* __restrict__ dst, gk::Geom g,
+                                const gk::DevTime* __restrict__ tm, int upload_step) {
+    const int nx4 = 2 * g.ng * g.ny, total = nx4 + 2 * g.ng * g.nx;
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= total) return;
+    int i, j;
+    if (id < nx4) {
+        const int side = id / (g.ng * g.ny), r = id - side * g.ng * g.ny;
+        j = g.jb + r / g.ng;
+        i = (side ? g.ie : 0) + r % g.ng;
+    } else {
+        const int m = id - nx4, side = m / (g.ng * g.nx), r = m - side * g.ng * g.nx;
+        j = (side ? g.je : 0) + r / g.nx;
+        i = g.ib + r % g.nx;
+    }
+    const double* src = donor && tm->step > upload_step ? donor : u;
+    dst[(long long)blockIdx.y * total + id] =
+        src[blockIdx.y * g.vstride + (long long)j * g.pitch + i];
+}
+inline dim3 rows_grid(const gk::Geom& g) {
+    return dim3((g.lenx + 255) / 256, (unsigned)std::min(5 * g.nzs * g.leny, 8192));
+}
+
+// A reference-layout host state into a device state buffer; its variable n
+// alone where n >= 0 (the rows of a variable's stored planes are equally
+// pitched, so each variable is one copy).
 int copy_ref_to_device(gk_handle* h, const double* ref, double* dev, int only = -1) {
     const gk::Geom& g = h->ctx.g;
     for (int n = 0; n < 5; ++n) {
         if (only >= 0 && n != only) continue;
-        for (int kk = 0; kk < g.nzs; ++kk) {
-            const int k = g.kofs + kk;
-            const double* src = ref + ((size_t)(n * g.lenz + k) * g.leny) * g.lenx;
-            double* dst = dev + (size_t)kSlotOf[n] * g.vstride + (size_t)kk * g.kstride;
-            GK_CUDA(h, cudaMemcpy2DAsync(dst, sizeof(double) * g.pitch, src, sizeof(double) * g.lenx,
-                                         sizeof(double) * g.lenx, g.leny, cudaMemcpyHostToDevice,
-                                         h->stream));
-        }
+        const double* src = ref + ((size_t)(n * g.lenz + g.kofs) * g.leny) * g.lenx;
+        GK_CUDA(h, cudaMemcpy2DAsync(dev + (size_t)kSlotOf[n] * g.vstride, sizeof(double) * g.pitch, src,
+                                     sizeof(double) * g.lenx, sizeof(double) * g.lenx,
+                                     (size_t)g.leny * g.nzs, cudaMemcpyHostToDevice, h->stream));
     }
     return GK_OK;
+}
+
+// The same into A through the scratch W: dense copies, unpacked by a kernel.
+int upload_dense(gk_handle* h, const double* ref) {
+    const gk::Geom& g = h->ctx.g;
+    const size_t len = (size_t)g.nzs * g.leny * g.lenx;
+    for (int n = 0; n < 5; ++n)
+        GK_CUDA(h, cudaMemcpyAsync(h->W + n * len, ref + ((size_t)(n * g.lenz + g.kofs) * g.leny) * g.lenx,
+                                   sizeof(double) * len, cudaMemcpyHostToDevice, h->stream));
+    k_unpack_state<<<rows_grid(g), 256, 0, h->stream>>>(h->W, h->A, g);
+    GK_CUDA(h, cudaGetLastError());
+    return GK_OK;
+}
+
+// Resets the step machinery at an upload; the clock (t, step, isContinue) is kept.
+__global__ void k_upload_reset(gk::DevTime* tm) {
+    tm->cmax_acc = (unsigned long long)__double_as_longlong(1e-16);
+    tm->floor_den = 0;
+    tm->floor_pre = 0;
+    tm->done_ctas = 0;
+    tm->status = 0;
+    tm->nlog = 0;
+    tm->active = 0;
 }
 
 // Whether every one of the n doubles at p has the bit pattern of +0.0; a
 // few host threads share the scan (it runs while the other planes copy).
 bool host_all_zero(const double* p, size_t n) {
+    // a thread costs about as much to start as it takes to scan 2^18 doubles
     const unsigned hw = std::thread::hardware_concurrency();
-    const size_t parts = std::max<size_t>(1, std::min<size_t>(hw ? hw : 1, 8));
+    const size_t parts = std::max<size_t>(1, std::min<size_t>({hw ? hw : 1u, 8, n >> 18}));
     std::vector<unsigned char> zero(parts, 1);
     auto scan = [&](size_t part) {
         const size_t lo = n * part / parts, hi = n * (part + 1) / parts;
@@ -773,13 +877,15 @@ void gk_destroy(gk_handle* h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->gexec) cudaGraphExecDestroy(h->gexec);
-    for (double* p : {h->A, h->B, h->C, h->W, h->F1, h->F2, h->F3, h->dlog, h->fixed}) cudaFree(p);
+    for (double* p : {h->A, h->B, h->C, h->W, h->F1, h->F2, h->F3, h->dlog, h->fixed, h->dstrips})
+        cudaFree(p);
     cudaFree(h->model);
     cudaFree(h->fired);
     cudaFree(h->shells);
     cudaFree(h->tm);
     cudaFree(h->dflag);
     if (h->htm) cudaFreeHost(h->htm);
+    if (h->hstrips) cudaFreeHost(h->hstrips);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -817,7 +923,8 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
             if (rc != GK_OK) return rc;
         }
     } else {
-        int rc0 = copy_ref_to_device(h, cons, h->A);
+        int rc0 = alloc_generic(h);  // 3D runs the 3D stage or the generic path
+        if (rc0 == GK_OK) rc0 = upload_dense(h, cons);
         if (rc0 != GK_OK) return rc0;
     }
     // Path: the fused kernel evolves four variables; it applies when the run
@@ -850,20 +957,8 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
         int rc = alloc_generic(h);
         if (rc != GK_OK) return rc;
     }
-    // reset the step machinery; the clock (t, step, isContinue) is kept
-    int rc = pull_time(h);
-    if (rc != GK_OK) return rc;
-    gk::DevTime t = *h->htm;
-    double seed = 1e-16;
-    std::memcpy(&t.cmax_acc, &seed, sizeof(double));
-    t.floor_den = 0;
-    t.floor_pre = 0;
-    t.done_ctas = 0;
-    t.status = 0;
-    t.nlog = 0;
-    t.active = 0;
-    *h->htm = t;
-    GK_CUDA(h, cudaMemcpyAsync(h->tm, h->htm, sizeof(gk::DevTime), cudaMemcpyHostToDevice, h->stream));
+    k_upload_reset<<<1, 1, 0, h->stream>>>(h->tm);
+    int rc;
     h->ks->cfl(h->ctx, h->A, 0, h->stream);
     GK_CUDA(h, cudaGetLastError());
     rc = pull_time(h);
@@ -879,83 +974,47 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
     int rc = check_ready(h);
     if (rc != GK_OK) return rc;
     if (!cons) return GK_ERR_INVALID;
-    rc = pull_time(h);
-    if (rc != GK_OK) return rc;
     const gk::Geom& g = h->ctx.g;
+    const int integ = h->ctx.ph.integrator;
     // The fused 2D path never writes MTZ, so a plane cleared at upload is
     // still +0.0 everywhere (no fixed data can fill its ghosts): a planes-only
     // download leaves the caller's plane as it is.
     const bool skip_mtz = !zero_other_planes && h->mtz_plane_zero && h->path == 1 &&
                           !h->ctx.ph.fixed_bd;
+    // Whose ghost strips the frame carries (k_pack_state): the stage buffer's
+    // (B, or C for the fused RK3 paths).  Euler runs in place and 1D y rows
+    // follow the reference's in-place order, so both keep A's.
+    const double* donor = nullptr;
+    if (integ != 1) donor = ((h->path == 1 || h->path == 2) && integ == 3) ? h->C : h->B;
+    const size_t len = (size_t)g.nzs * g.leny * g.lenx, total = g.ndim == 2 ? strip_doubles(g) : 0;
+    const bool dense = h->path != 1;
+    const int slots = skip_mtz ? 4 : 5;  // MTZ's is the last
     h->io_down = 0;
+    if (dense) {
+        k_pack_state<<<rows_grid(g), 256, 0, h->stream>>>(h->A, donor, h->W, g, h->ctx.ph.fill_z, h->tm,
+                                                          h->upload_step);
+    } else {
+        k_gather_strips<<<dim3((unsigned)((total + 127) / 128), slots), 128, 0, h->stream>>>(
+            h->A, donor, h->dstrips, g, h->tm, h->upload_step);
+    }
+    GK_CUDA(h, cudaGetLastError());
     for (int n = 0; n < 5; ++n) {
         if (skip_mtz && n == 3) continue;
-        for (int kk = 0; kk < g.nzs; ++kk) {
-            const int k = g.kofs + kk;
-            double* dst = cons + ((size_t)(n * g.lenz + k) * g.leny) * g.lenx;
-            const double* src = h->A + (size_t)kSlotOf[n] * g.vstride + (size_t)kk * g.kstride;
-            GK_CUDA(h, cudaMemcpy2DAsync(dst, sizeof(double) * g.lenx, src, sizeof(double) * g.pitch,
+        double* dst = cons + ((size_t)(n * g.lenz + g.kofs) * g.leny) * g.lenx;
+        if (dense)
+            GK_CUDA(h, cudaMemcpyAsync(dst, h->W + n * len, sizeof(double) * len, cudaMemcpyDeviceToHost,
+                                       h->stream));
+        else
+            GK_CUDA(h, cudaMemcpy2DAsync(dst, sizeof(double) * g.lenx,
+                                         h->A + (size_t)kSlotOf[n] * g.vstride, sizeof(double) * g.pitch,
                                          sizeof(double) * g.lenx, g.leny, cudaMemcpyDeviceToHost,
                                          h->stream));
-            h->io_down += (long long)sizeof(double) * g.lenx * g.leny;
-        }
+        h->io_down += (long long)(sizeof(double) * len);
     }
-    // Ghost strips as the reference leaves them after a step: Sim's integrators
-    // end with cons.Swap(consTemp) (rk2.cpp:21, rk3.cpp:27), so the written
-    // array carries the ghost fill of the last intermediate stage state.  That
-    // fill sits in the stage buffer (B, or C for the fused RK3 path); the
-    // strips of active rows/columns are taken from there.  Euler runs in place
-    // and 1D y rows follow the reference's in-place order, so both keep A's.
-    const double* donor = nullptr;
-    if (h->htm->step > h->upload_step && h->ctx.ph.integrator != 1)
-        donor = ((h->path == 1 || h->path == 2) && h->ctx.ph.integrator == 3) ? h->C : h->B;
-    if (donor) {
-        const size_t rowb = sizeof(double) * g.lenx, prow = sizeof(double) * g.pitch;
-        for (int n = 0; n < 5; ++n) {
-            if (skip_mtz && n == 3) continue;
-            for (int kk = 0; kk < g.nzs; ++kk) {
-                const int k = g.kofs + kk;
-                if (k < g.kb || k >= g.ke) continue;
-                double* dst = cons + ((size_t)(n * g.lenz + k) * g.leny) * g.lenx;
-                const double* src = donor + (size_t)kSlotOf[n] * g.vstride + (size_t)kk * g.kstride;
-                if (g.nx > 1) {
-                    for (int side = 0; side < 2; ++side) {
-                        const int i0 = side == 0 ? 0 : g.ie;
-                        GK_CUDA(h, cudaMemcpy2DAsync(dst + (size_t)g.jb * g.lenx + i0, rowb,
-                                                     src + (size_t)g.jb * g.pitch + i0, prow,
-                                                     sizeof(double) * g.ng, g.ny,
-                                                     cudaMemcpyDeviceToHost, h->stream));
-                        h->io_down += (long long)sizeof(double) * g.ng * g.ny;
-                    }
-                }
-                if (g.ny > 1) {
-                    for (int side = 0; side < 2; ++side) {
-                        const int j0 = side == 0 ? 0 : g.je;
-                        GK_CUDA(h, cudaMemcpy2DAsync(dst + (size_t)j0 * g.lenx + g.ib, rowb,
-                                                     src + (size_t)j0 * g.pitch + g.ib, prow,
-                                                     sizeof(double) * g.nx, g.ng,
-                                                     cudaMemcpyDeviceToHost, h->stream));
-                        h->io_down += (long long)sizeof(double) * g.nx * g.ng;
-                    }
-                }
-            }
-            if (g.nz > 1) {
-                for (int side = 0; side < 2; ++side) {
-                    if (!((h->ctx.ph.fill_z >> side) & 1)) continue;
-                    for (int gi = 0; gi < g.ng; ++gi) {
-                        const int k = side == 0 ? gi : g.ke + gi;
-                        double* dst = cons + ((size_t)(n * g.lenz + k) * g.leny) * g.lenx;
-                        const double* src = donor + (size_t)kSlotOf[n] * g.vstride +
-                                            (size_t)(k - g.kofs) * g.kstride;
-                        GK_CUDA(h, cudaMemcpy2DAsync(dst + (size_t)g.jb * g.lenx + g.ib, rowb,
-                                                     src + (size_t)g.jb * g.pitch + g.ib, prow,
-                                                     sizeof(double) * g.nx, g.ny,
-                                                     cudaMemcpyDeviceToHost, h->stream));
-                        h->io_down += (long long)sizeof(double) * g.nx * g.ny;
-                    }
-                }
-            }
-        }
+    if (!dense) {
+        GK_CUDA(h, cudaMemcpyAsync(h->hstrips, h->dstrips, sizeof(double) * slots * total,
+                                   cudaMemcpyDeviceToHost, h->stream));
+        h->io_down += (long long)(sizeof(double) * slots * total);
     }
     if (g.nzs == 1 && zero_other_planes) {
         const size_t plane = (size_t)g.leny * g.lenx;
@@ -963,7 +1022,20 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
             for (int k = 0; k < g.lenz; ++k)
                 if (k != g.kofs) std::memset(cons + (size_t)(n * g.lenz + k) * plane, 0, plane * sizeof(double));
     }
-    GK_CUDA(h, cudaStreamSynchronize(h->stream));
+    rc = pull_time(h);  // and the copies
+    if (rc != GK_OK || dense) return rc;
+    for (int n = 0; n < 5; ++n) {
+        if (skip_mtz && n == 3) continue;
+        double* dst = cons + ((size_t)(n * g.lenz + g.kofs) * g.leny) * g.lenx;
+        const double* src = h->hstrips + kSlotOf[n] * total;
+        for (int side = 0; side < 2; ++side)
+            for (int j = g.jb; j < g.je; ++j)
+                for (int q = 0; q < g.ng; ++q) dst[(size_t)j * g.lenx + (side ? g.ie : 0) + q] = *src++;
+        for (int side = 0; side < 2; ++side)
+            for (int q = 0; q < g.ng; ++q, src += g.nx)
+                std::memcpy(dst + (size_t)((side ? g.je : 0) + q) * g.lenx + g.ib, src,
+                            sizeof(double) * g.nx);
+    }
     return GK_OK;
 }
 
