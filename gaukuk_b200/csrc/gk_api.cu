@@ -504,6 +504,21 @@ int run_host_fills(gk_handle* h, double* u) {
     return GK_OK;
 }
 
+// Whether a 2D run on the generic path takes the five-variable x-y stage
+// (k_stage3d without z fluxes): RK2 and RK3; forward Euler updates in place,
+// and the learned correction as a pass needs the face-flux arrays.
+bool stage5_2d(const gk_handle* h) {
+    return h->path == 0 && h->ctx.g.ndim == 2 && h->ctx.ph.integrator != 1 && !h->model;
+}
+
+// The buffer whose ghost fill a written frame carries (k_pack_state): the last
+// intermediate stage state's (B, or C where RK3's second stage lands in C).
+// Euler runs in place and keeps A's.
+const double* last_stage_buffer(const gk_handle* h) {
+    if (h->ctx.ph.integrator == 1) return nullptr;
+    return h->ctx.ph.integrator == 3 && (h->path == 1 || h->path == 2 || stage5_2d(h)) ? h->C : h->B;
+}
+
 // One time step.  Kernel order per RK stage follows Sim::RK2_/RK3_/
 // ForwardEuler_ (rk2.cpp:11-23, rk3.cpp:11-29, forward_euler.cpp:11-18),
 // wrapped in the Strang half kicks of sim.cpp:85-91; the step ends with the
@@ -542,25 +557,27 @@ void enqueue_step(gk_handle* h, Profiler* prof) {
         GK_L(gk::K_STAGE, k.run1d(c, A, B, 1, s));
         return;
     }
-    if (h->path == 2) {
-        // z fluxes of the stage's state into F3, then the fused x-y stage;
-        // without a kick after it the last stage also reduces the CFL speed
-        const bool kicks = c.ph.has_grav || c.ph.npoint;
-        const int last = kicks ? 1 : 2;
-        GK_L(gk::K_BC, fill(A));
-        GK_L(gk::K_FLUX, k.zflux(c, A, h->F3, s));
-        GK_L(gk::K_STAGE, k.stage3d(c, A, nullptr, B, h->F3, 0, 1.0, 1.0, 0.0, s));
-        GK_L(gk::K_BC, fill(B));
-        GK_L(gk::K_FLUX, k.zflux(c, B, h->F3, s));
+    if (h->path == 2 || stage5_2d(h)) {
+        // 3D: z fluxes of the stage's state into F3, then the fused x-y stage;
+        // 2D with five variables: the x-y stage alone.  The last stage also
+        // applies the second half kick (a binary's, with its sine and cosine,
+        // is a pass of its own), the CFL reduction and the step epilogue.
+        const bool kicks = c.ph.has_grav || c.ph.npoint, binary = c.ph.npoint == 2;
+        const int last = binary ? 0 : (kicks ? 2 : 1);
+        auto stage = [&](double* uc, const double* u0, double* out, int la, double c1, double c2,
+                         double c3) {
+            GK_L(gk::K_BC, fill(uc));
+            if (h->path == 2) GK_L(gk::K_FLUX, k.zflux(c, uc, h->F3, s));
+            GK_L(gk::K_STAGE, k.stage3d(c, uc, u0, out, h->F3, u0 != nullptr, la, c1, c2, c3, s));
+        };
+        stage(A, nullptr, B, 0, 1.0, 1.0, 0.0);
         if (integ == 3) {
-            GK_L(gk::K_STAGE, k.stage3d(c, B, A, Cb, h->F3, 1, 0.75, 0.25, 0.25, s));
-            GK_L(gk::K_BC, fill(Cb));
-            GK_L(gk::K_FLUX, k.zflux(c, Cb, h->F3, s));
-            GK_L(gk::K_STAGE, k.stage3d(c, Cb, A, A, h->F3, last, frac13, 2 * frac13, 2 * frac13, s));
+            stage(B, A, Cb, 0, 0.75, 0.25, 0.25);
+            stage(Cb, A, A, last, frac13, 2 * frac13, 2 * frac13);
         } else {
-            GK_L(gk::K_STAGE, k.stage3d(c, B, A, A, h->F3, last, 0.5, 0.5, 0.5, s));
+            stage(B, A, A, last, 0.5, 0.5, 0.5);
         }
-        if (kicks) {
+        if (binary) {
             GK_L(gk::K_KICK, k.kick(c, A, 1, s));
             GK_L(gk::K_CFL, k.cfl(c, A, 1, s));
         }
@@ -975,17 +992,14 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
     if (rc != GK_OK) return rc;
     if (!cons) return GK_ERR_INVALID;
     const gk::Geom& g = h->ctx.g;
-    const int integ = h->ctx.ph.integrator;
     // The fused 2D path never writes MTZ, so a plane cleared at upload is
     // still +0.0 everywhere (no fixed data can fill its ghosts): a planes-only
     // download leaves the caller's plane as it is.
     const bool skip_mtz = !zero_other_planes && h->mtz_plane_zero && h->path == 1 &&
                           !h->ctx.ph.fixed_bd;
-    // Whose ghost strips the frame carries (k_pack_state): the stage buffer's
-    // (B, or C for the fused RK3 paths).  Euler runs in place and 1D y rows
-    // follow the reference's in-place order, so both keep A's.
-    const double* donor = nullptr;
-    if (integ != 1) donor = ((h->path == 1 || h->path == 2) && integ == 3) ? h->C : h->B;
+    // whose ghost strips the frame carries; 1D y rows follow the reference's
+    // in-place order and keep A's (from_donor)
+    const double* donor = last_stage_buffer(h);
     const size_t len = (size_t)g.nzs * g.leny * g.lenx, total = g.ndim == 2 ? strip_doubles(g) : 0;
     const bool dense = h->path != 1;
     const int slots = skip_mtz ? 4 : 5;  // MTZ's is the last
@@ -1221,8 +1235,10 @@ int gk_graph_info(gk_handle* h, int* steps_per_graph, int* launches_per_step) {
     if (h->path == 1) {
         // kick, (ghost fill + stage) per stage; with periodic images the stage alone
         per = (c.ph.has_grav ? 1 : 0) + (c.ph.periodic_images ? 1 : 2 + inner) * stages;
-    } else if (h->path == 2) {
-        per = (c.ph.has_grav || c.ph.npoint ? 3 : 0) + (3 + inner) * stages;
+    } else if (h->path == 2 || stage5_2d(h)) {
+        // first kick, (ghost fill, z fluxes, stage) per stage; a binary's second kick and CFL
+        per = (c.ph.has_grav || c.ph.npoint ? 1 : 0) + ((h->path == 2 ? 3 : 2) + inner) * stages +
+              (c.ph.npoint == 2 ? 2 : 0);
     } else if (h->path == 3) {
         per = 1;  // in a graph, one launch runs all of its steps
     } else {

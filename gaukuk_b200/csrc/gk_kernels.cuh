@@ -479,24 +479,19 @@ __global__ void k_update(const double* u0, const double* uc, double* out,
 // mass (point_gravity.cpp:11-92) or two (binary_gravity.cpp), whose second
 // mass orbits at angle omega*t + theta1 with t = t_n + dt/2 for the first
 // half kick (which = 0) and t_n + dt for the second (which = 1).
-__global__ void k_kick(double* __restrict__ u, Geom g, Phys ph, const DevTime* __restrict__ tm,
-                       int which) {
-    if (!tm->active) return;
-    const int i = g.ib + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = g.jb + blockIdx.y;
-    const int k = g.kb + blockIdx.z;
-    if (i >= g.ie) return;
-    const double hdt = 0.5 * tm->dt;
-    const long long c = sidx(g, k, j, i);
+// The half kick of one cell's state r (slots DEN, MTX, MTY, ENG, MTZ).
+// BINARY = false: at most one point mass (the orbit's sine and cosine stay out).
+template <bool BINARY>
+__device__ __forceinline__ void kick_cell(double (&r)[5], const Geom& g, const Phys& ph, double dt,
+                                          double tnow, int which, int i, int j, int k) {
+    const double hdt = 0.5 * dt;
     const int moms[3] = {gk::S_MTX, gk::S_MTY, gk::S_MTZ};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double gd = ph.grav[d];
         if (gd == 0) continue;
-        double& E = u[gk::S_ENG * g.vstride + c];
-        double& m = u[moms[d] * g.vstride + c];
-        E += m * gd * hdt;
-        m += u[gk::S_DEN * g.vstride + c] * gd * hdt;
+        r[gk::S_ENG] += r[moms[d]] * gd * hdt;
+        r[moms[d]] += r[gk::S_DEN] * gd * hdt;
     }
     if (ph.npoint == 0) return;
     const double xnow = centre(g.xmin, g.ng, g.dx, i);
@@ -512,8 +507,8 @@ __global__ void k_kick(double* __restrict__ u, Geom g, Phys ph, const DevTime* _
         gxdt = gv * delx;
         gydt = gv * dely;
         gzdt = gv * delz;
-        if (ph.npoint == 2) {
-            const double t = which == 0 ? tm->t + 0.5 * tm->dt : tm->t + tm->dt;
+        if (BINARY && ph.npoint == 2) {
+            const double t = which == 0 ? tnow + 0.5 * dt : tnow + dt;
             const double theta = ph.pm[8] * t + ph.pm[10];
             const double x1 = ph.pm[9] * cos(theta), y1 = ph.pm[9] * sin(theta), z1 = ph.pm[6];
             const double dx1 = xnow - x1, dy1 = ynow - y1, dz1 = znow - z1;
@@ -527,15 +522,29 @@ __global__ void k_kick(double* __restrict__ u, Geom g, Phys ph, const DevTime* _
             gzdt = gv * delz + g1 * dz1 + gInd * z1;
         }
     }
-    double& D = u[gk::S_DEN * g.vstride + c];
-    double& E = u[gk::S_ENG * g.vstride + c];
-    double& MX = u[gk::S_MTX * g.vstride + c];
-    double& MY = u[gk::S_MTY * g.vstride + c];
-    double& MZ = u[gk::S_MTZ * g.vstride + c];
-    E += MX * gxdt + MY * gydt + MZ * gzdt;
-    MX += D * gxdt;
-    MY += D * gydt;
-    MZ += D * gzdt;
+    r[gk::S_ENG] += r[gk::S_MTX] * gxdt + r[gk::S_MTY] * gydt + r[gk::S_MTZ] * gzdt;
+    r[gk::S_MTX] += r[gk::S_DEN] * gxdt;
+    r[gk::S_MTY] += r[gk::S_DEN] * gydt;
+    r[gk::S_MTZ] += r[gk::S_DEN] * gzdt;
+}
+__global__ void k_kick(double* __restrict__ u, Geom g, Phys ph, const DevTime* __restrict__ tm,
+                       int which) {
+    if (!tm->active) return;
+    const int i = g.ib + blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = g.jb + blockIdx.y;
+    const int k = g.kb + blockIdx.z;
+    if (i >= g.ie) return;
+    const long long c = sidx(g, k, j, i);
+    // constant gravity along one axis touches that momentum only
+    const bool moves[5] = {true, ph.npoint || ph.grav[0] != 0, ph.npoint || ph.grav[1] != 0, true,
+                           ph.npoint || ph.grav[2] != 0};
+    double r[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) r[v] = moves[v] ? u[v * g.vstride + c] : 0.0;
+    kick_cell<true>(r, g, ph, tm->dt, tm->t, which, i, j, k);
+#pragma unroll
+    for (int v = 1; v < 5; ++v)
+        if (moves[v]) u[v * g.vstride + c] = r[v];
 }
 
 // ------------------------------------------------------------ CFL + epilogue
@@ -1825,34 +1834,55 @@ void launch_zflux(const Ctx& c, const double* u, double* F3, cudaStream_t s) {
     else k_zflux<false><<<grid, 128, 0, s>>>(u, F3, g, c.ph, c.tm, zseg);
 }
 
-template <int NT>
+// last: 0 a stage inside the step; 1 the step's last stage (CFL reduction and
+// epilogue); 2 the last stage with the second half kick before them.
+template <int NT, bool ZF>
 static void launch_stage3d_nt(const Ctx& c, const double* uc, const double* u0, double* out,
-                              const double* F3, int three, double c1, double c2, double c3,
-                              cudaStream_t s) {
+                              const double* F3, int rows, int three, int last, double c1, double c2,
+                              double c3, cudaStream_t s) {
     const Geom& g = c.g;
-    const int rows = stage3d_rows(g, NT);
+    const int has_z = c.has_vz || g.ndim == 3;
     dim3 grid((g.nx + NT - 5) / (NT - 4), (g.ny + rows - 1) / rows, g.nz);
 #define GK_S3(TH, PL, LA) \
-    k_stage3d<NT, TH, PL, LA><<<grid, NT, 0, s>>>(uc, u0, out, F3, g, c.ph, c1, c2, c3, c.tm, rows)
-    if (three == 2) {
-        if (c.ph.plm) GK_S3(true, true, true);
-        else GK_S3(true, false, true);
+    k_stage3d<NT, TH, PL, LA, ZF><<<grid, NT, 0, s>>>(uc, u0, out, F3, g, c.ph, c1, c2, c3, c.tm, rows, has_z)
+    if (last == 2) {
+        if (c.ph.plm) GK_S3(true, true, 2);
+        else GK_S3(true, false, 2);
+    } else if (last) {
+        if (c.ph.plm) GK_S3(true, true, 1);
+        else GK_S3(true, false, 1);
     } else if (three) {
-        if (c.ph.plm) GK_S3(true, true, false);
-        else GK_S3(true, false, false);
+        if (c.ph.plm) GK_S3(true, true, 0);
+        else GK_S3(true, false, 0);
     } else {
-        if (c.ph.plm) GK_S3(false, true, false);
-        else GK_S3(false, false, false);
+        if (c.ph.plm) GK_S3(false, true, 0);
+        else GK_S3(false, false, 0);
     }
 #undef GK_S3
 }
 
 void launch_stage3d(const Ctx& c, const double* uc, const double* u0, double* out, const double* F3,
-                    int three, double c1, double c2, double c3, cudaStream_t s) {
-    switch (stage3d_nt(c.g)) {
-        case 64: launch_stage3d_nt<64>(c, uc, u0, out, F3, three, c1, c2, c3, s); break;
-        case 96: launch_stage3d_nt<96>(c, uc, u0, out, F3, three, c1, c2, c3, s); break;
-        default: launch_stage3d_nt<128>(c, uc, u0, out, F3, three, c1, c2, c3, s); break;
+                    int three, int last, double c1, double c2, double c3, cudaStream_t s) {
+    const Geom& g = c.g;
+    if (g.ndim == 2) {
+        // CTAs of 64 threads where they finish the plane in fewer row times
+        const int r64 = stage3d_rows(g, 64), r128 = stage3d_rows(g, 128);
+        auto cost = [&](int nt, int rows) {
+            const long long ctas = (long long)((g.nx + nt - 5) / (nt - 4)) * ((g.ny + rows - 1) / rows);
+            const long long slots = 148LL * (kStage3dThreadsPerSM / nt);
+            return (double)((ctas + slots - 1) / slots) * (rows + 2.5);
+        };
+        if (cost(64, r64) < cost(128, r128))
+            launch_stage3d_nt<64, false>(c, uc, u0, out, F3, r64, three, last, c1, c2, c3, s);
+        else
+            launch_stage3d_nt<128, false>(c, uc, u0, out, F3, r128, three, last, c1, c2, c3, s);
+        return;
+    }
+    const int nt = stage3d_nt(g), rows = stage3d_rows(g, nt);
+    switch (nt) {
+        case 64: launch_stage3d_nt<64, true>(c, uc, u0, out, F3, rows, three, last, c1, c2, c3, s); break;
+        case 96: launch_stage3d_nt<96, true>(c, uc, u0, out, F3, rows, three, last, c1, c2, c3, s); break;
+        default: launch_stage3d_nt<128, true>(c, uc, u0, out, F3, rows, three, last, c1, c2, c3, s); break;
     }
 }
 

@@ -212,11 +212,16 @@ __global__ void __launch_bounds__(128)
 // against 207); fast mode at 512 threads ran 2.28 -> 2.42 ms at 256^3 (its
 // early loads need the registers).
 constexpr int kStage3dThreadsPerSM = 384;
-template <int NT, bool THREE, bool PLM, bool LAST>
+// ZF = false: a 2D run with all five variables (one plane, no z fluxes): the
+// update is k_update's 2D expression.  A 2D run off the four-variable path
+// (v_z, z gravity, point masses, an immersed body) took five launches per
+// stage through primitive and flux arrays; this is one.
+// LAST = 2: the second half kick of constant gravity and one point mass too.
+template <int NT, bool THREE, bool PLM, int LAST, bool ZF>
 __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
     k_stage3d(const double* __restrict__ uc, const double* u0, double* out,
               const double* __restrict__ F3, Geom g, Phys ph, double c1, double c2, double c3,
-              DevTime* tm, int rows) {
+              DevTime* tm, int rows, int has_z) {
     if (!tm->active) return;
     unsigned long long cbest = 0ull;  // CFL speed of this thread's cells (bit pattern)
     __shared__ double sP[5][NT];
@@ -272,12 +277,14 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
         double zlo[5], zhi[5], b0[5];
         constexpr bool kEarly = GK_FASTMATH;
         auto load_row_inputs = [&]() {
-            const long long fc = fidx(g, k, f - 1, xi);
+            const long long fc = ZF ? fidx(g, k, f - 1, xi) : 0;
             const long long c = at(f - 1);
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
-                zlo[v] = __ldg(F3 + v * g.fvstride + fc);
-                zhi[v] = __ldg(F3 + v * g.fvstride + fc + g.fkstride);
+                if (ZF) {
+                    zlo[v] = __ldg(F3 + v * g.fvstride + fc);
+                    zhi[v] = __ldg(F3 + v * g.fvstride + fc + g.fkstride);
+                }
                 b0[v] = THREE ? u0[v * g.vstride + c] : uc[v * g.vstride + c];
             }
         };
@@ -339,14 +346,16 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
                 double dF = (sF[v][tr] - fx[v]) * dtdx;
-                dF = dF + (fy[v] - fyPrev[v]) * dtdy + (zhi[v] - zlo[v]) * dtdz;
+                if (ZF) dF = dF + (fy[v] - fyPrev[v]) * dtdy + (zhi[v] - zlo[v]) * dtdz;
+                else dF = dF + (fy[v] - fyPrev[v]) * dtdy;
                 if (THREE) r[v] = c1 * b0[v] + c2 * uc[v * g.vstride + c] - c3 * dF;
                 else r[v] = c1 * b0[v] - c2 * dF;
             }
             floors5(r, ph, tm);
             if (LAST) {
+                if (LAST == 2) kick_cell<false>(r, g, ph, dt, tm->t, 1, xi, f - 1, k);
                 const double local = cell_cmax(r[gk::S_DEN], r[gk::S_MTX], r[gk::S_MTY],
-                                               r[gk::S_MTZ], r[gk::S_ENG], ph, true);
+                                               r[gk::S_MTZ], r[gk::S_ENG], ph, ZF || has_z);
                 const unsigned long long b = (unsigned long long)__double_as_longlong(local);
                 cbest = b > cbest ? b : cbest;
             }
@@ -360,7 +369,8 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
         }
         Pm1 = P0;
         P0 = P1;
-    }    if (LAST) {
+    }
+    if (LAST) {
         __shared__ unsigned long long wmax[NT / 32];
         __shared__ int last;
 #pragma unroll
