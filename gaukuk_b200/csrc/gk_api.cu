@@ -127,6 +127,7 @@ struct gk_handle {
     int* dflag = nullptr;
     double* dstrips = nullptr;  // 2D: a download's ghost strips, gathered (device),
     double* hstrips = nullptr;  // and their pinned landing place
+    cudaEvent_t copied[5] = {};  // a variable's plane is in the caller's array
     int path = 0;  // 0 generic, 1 fused 2D
     bool uploaded = false;
     int upload_step = 0;  // clock step at the last upload
@@ -300,6 +301,7 @@ int alloc_state(gk_handle* h) {
         const size_t sb = sizeof(double) * 5 * strip_doubles(g);
         GK_CUDA(h, cudaMalloc(&h->dstrips, sb));
         GK_CUDA(h, cudaMallocHost(&h->hstrips, sb));
+        for (cudaEvent_t& e : h->copied) GK_CUDA(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     gk::DevTime t{};
     t.t = 0; t.dt = 1e10; t.tNext = 0; t.dtUntilOutput = 1e10;  // sim.cpp:45-46
@@ -903,6 +905,8 @@ void gk_destroy(gk_handle* h) {
     cudaFree(h->dflag);
     if (h->htm) cudaFreeHost(h->htm);
     if (h->hstrips) cudaFreeHost(h->hstrips);
+    for (cudaEvent_t e : h->copied)
+        if (e) cudaEventDestroy(e);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -1012,23 +1016,25 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
             h->A, donor, h->dstrips, g, h->tm, h->upload_step);
     }
     GK_CUDA(h, cudaGetLastError());
-    for (int n = 0; n < 5; ++n) {
-        if (skip_mtz && n == 3) continue;
-        double* dst = cons + ((size_t)(n * g.lenz + g.kofs) * g.leny) * g.lenx;
-        if (dense)
-            GK_CUDA(h, cudaMemcpyAsync(dst, h->W + n * len, sizeof(double) * len, cudaMemcpyDeviceToHost,
-                                       h->stream));
-        else
-            GK_CUDA(h, cudaMemcpy2DAsync(dst, sizeof(double) * g.lenx,
-                                         h->A + (size_t)kSlotOf[n] * g.vstride, sizeof(double) * g.pitch,
-                                         sizeof(double) * g.lenx, g.leny, cudaMemcpyDeviceToHost,
-                                         h->stream));
-        h->io_down += (long long)(sizeof(double) * len);
-    }
     if (!dense) {
         GK_CUDA(h, cudaMemcpyAsync(h->hstrips, h->dstrips, sizeof(double) * slots * total,
                                    cudaMemcpyDeviceToHost, h->stream));
         h->io_down += (long long)(sizeof(double) * slots * total);
+    }
+    for (int n = 0; n < 5; ++n) {
+        if (skip_mtz && n == 3) continue;
+        double* dst = cons + ((size_t)(n * g.lenz + g.kofs) * g.leny) * g.lenx;
+        if (dense) {
+            GK_CUDA(h, cudaMemcpyAsync(dst, h->W + n * len, sizeof(double) * len, cudaMemcpyDeviceToHost,
+                                       h->stream));
+        } else {
+            GK_CUDA(h, cudaMemcpy2DAsync(dst, sizeof(double) * g.lenx,
+                                         h->A + (size_t)kSlotOf[n] * g.vstride, sizeof(double) * g.pitch,
+                                         sizeof(double) * g.lenx, g.leny, cudaMemcpyDeviceToHost,
+                                         h->stream));
+            GK_CUDA(h, cudaEventRecord(h->copied[n], h->stream));
+        }
+        h->io_down += (long long)(sizeof(double) * len);
     }
     if (g.nzs == 1 && zero_other_planes) {
         const size_t plane = (size_t)g.leny * g.lenx;
@@ -1036,10 +1042,10 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
             for (int k = 0; k < g.lenz; ++k)
                 if (k != g.kofs) std::memset(cons + (size_t)(n * g.lenz + k) * plane, 0, plane * sizeof(double));
     }
-    rc = pull_time(h);  // and the copies
-    if (rc != GK_OK || dense) return rc;
-    for (int n = 0; n < 5; ++n) {
+    // the strips of a variable go in while the next variables still copy
+    for (int n = 0; n < 5 && !dense; ++n) {
         if (skip_mtz && n == 3) continue;
+        GK_CUDA(h, cudaEventSynchronize(h->copied[n]));
         double* dst = cons + ((size_t)(n * g.lenz + g.kofs) * g.leny) * g.lenx;
         const double* src = h->hstrips + kSlotOf[n] * total;
         for (int side = 0; side < 2; ++side)
@@ -1050,7 +1056,7 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
                 std::memcpy(dst + (size_t)((side ? g.je : 0) + q) * g.lenx + g.ib, src,
                             sizeof(double) * g.nx);
     }
-    return GK_OK;
+    return pull_time(h);  // and the copies
 }
 
 int gk_download_cons(gk_handle* h, double* cons) { return download(h, cons, true); }
