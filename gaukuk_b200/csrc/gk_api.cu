@@ -79,6 +79,7 @@ struct KernelSet {
     decltype(&gk_parity::launch_epilogue) epilogue;
     decltype(&gk_parity::launch_stage2d_learn) stage2d_learn;
     decltype(&gk_parity::launch_run1d) run1d;
+    decltype(&gk_parity::launch_row_stage) row_stage;
 };
 
 const KernelSet kParity = {gk_parity::launch_bc,     gk_parity::launch_c2p,
@@ -89,13 +90,14 @@ const KernelSet kParity = {gk_parity::launch_bc,     gk_parity::launch_c2p,
                            gk_parity::launch_ens_bc,  gk_parity::launch_ens_begin,
                            gk_parity::launch_zflux,   gk_parity::launch_stage3d,
                            gk_parity::launch_epilogue, gk_parity::launch_stage2d_learn,
-                           gk_parity::launch_run1d};
+                           gk_parity::launch_run1d, gk_parity::launch_row_stage};
 const KernelSet kFast = {gk_fast::launch_bc,     gk_fast::launch_c2p,     gk_fast::launch_flux,
                          gk_fast::launch_update, gk_fast::launch_kick,    gk_fast::launch_cfl,
                          gk_fast::launch_stage2d, gk_fast::launch_begin,  gk_fast::launch_mtz_check,
                          gk_fast::launch_ens_stage, gk_fast::launch_ens_bc, gk_fast::launch_ens_begin,
                          gk_fast::launch_zflux, gk_fast::launch_stage3d, gk_fast::launch_epilogue,
-                         gk_fast::launch_stage2d_learn, gk_fast::launch_run1d};
+                         gk_fast::launch_stage2d_learn, gk_fast::launch_run1d,
+                         gk_fast::launch_row_stage};
 
 constexpr int kLogCap = 1 << 20;
 
@@ -506,11 +508,12 @@ int run_host_fills(gk_handle* h, double* u) {
     return GK_OK;
 }
 
-// Whether a 2D run on the generic path takes the five-variable x-y stage
-// (k_stage3d without z fluxes): RK2 and RK3; forward Euler updates in place,
-// and the learned correction as a pass needs the face-flux arrays.
-bool stage5_2d(const gk_handle* h) {
-    return h->path == 0 && h->ctx.g.ndim == 2 && h->ctx.ph.integrator != 1 && !h->model;
+// Whether a run on the generic path takes a fused stage of five variables: in
+// 2D the x-y stage without z fluxes (k_stage3d), in 1D the row stage
+// (k_row_stage).  RK2 and RK3; forward Euler updates in place, and the learned
+// correction as a pass needs the face-flux arrays.
+bool fused5(const gk_handle* h) {
+    return h->path == 0 && h->ctx.g.ndim <= 2 && h->ctx.ph.integrator != 1 && !h->model;
 }
 
 // The buffer whose ghost fill a written frame carries (k_pack_state): the last
@@ -518,7 +521,7 @@ bool stage5_2d(const gk_handle* h) {
 // Euler runs in place and keeps A's.
 const double* last_stage_buffer(const gk_handle* h) {
     if (h->ctx.ph.integrator == 1) return nullptr;
-    return h->ctx.ph.integrator == 3 && (h->path == 1 || h->path == 2 || stage5_2d(h)) ? h->C : h->B;
+    return h->ctx.ph.integrator == 3 && (h->path == 1 || h->path == 2 || fused5(h)) ? h->C : h->B;
 }
 
 // One time step.  Kernel order per RK stage follows Sim::RK2_/RK3_/
@@ -559,15 +562,21 @@ void enqueue_step(gk_handle* h, Profiler* prof) {
         GK_L(gk::K_STAGE, k.run1d(c, A, B, 1, s));
         return;
     }
-    if (h->path == 2 || stage5_2d(h)) {
+    if (h->path == 2 || fused5(h)) {
         // 3D: z fluxes of the stage's state into F3, then the fused x-y stage;
-        // 2D with five variables: the x-y stage alone.  The last stage also
+        // 2D with five variables: the x-y stage alone; 1D: the row stage, which
+        // fills its own ghosts.  The last stage also
         // applies the second half kick (a binary's, with its sine and cosine,
         // is a pass of its own), the CFL reduction and the step epilogue.
         const bool kicks = c.ph.has_grav || c.ph.npoint, binary = c.ph.npoint == 2;
         const int last = binary ? 0 : (kicks ? 2 : 1);
         auto stage = [&](double* uc, const double* u0, double* out, int la, double c1, double c2,
                          double c3) {
+            if (c.g.ndim == 1) {
+                if (!h->host_fills.empty()) GK_L(gk::K_BC, fill(uc));
+                GK_L(gk::K_STAGE, k.row_stage(c, uc, u0, out, la, c1, c2, c3, s));
+                return;
+            }
             GK_L(gk::K_BC, fill(uc));
             if (h->path == 2) GK_L(gk::K_FLUX, k.zflux(c, uc, h->F3, s));
             GK_L(gk::K_STAGE, k.stage3d(c, uc, u0, out, h->F3, u0 != nullptr, la, c1, c2, c3, s));
@@ -1241,9 +1250,11 @@ int gk_graph_info(gk_handle* h, int* steps_per_graph, int* launches_per_step) {
     if (h->path == 1) {
         // kick, (ghost fill + stage) per stage; with periodic images the stage alone
         per = (c.ph.has_grav ? 1 : 0) + (c.ph.periodic_images ? 1 : 2 + inner) * stages;
-    } else if (h->path == 2 || stage5_2d(h)) {
+    } else if (h->path == 2 || fused5(h)) {
         // first kick, (ghost fill, z fluxes, stage) per stage; a binary's second kick and CFL
-        per = (c.ph.has_grav || c.ph.npoint ? 1 : 0) + ((h->path == 2 ? 3 : 2) + inner) * stages +
+        // (1D: the stage alone)
+        const int each = c.g.ndim == 1 ? 1 : (h->path == 2 ? 3 : 2) + inner;
+        per = (c.ph.has_grav || c.ph.npoint ? 1 : 0) + each * stages +
               (c.ph.npoint == 2 ? 2 : 0);
     } else if (h->path == 3) {
         per = 1;  // in a graph, one launch runs all of its steps

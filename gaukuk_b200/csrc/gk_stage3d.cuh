@@ -199,6 +199,35 @@ __global__ void __launch_bounds__(128)
     }
 }
 
+// The end of a step's last stage: the CTA's largest CFL speed (bit pattern)
+// into the clock; the last of `ctas` CTAs runs the step epilogue.
+template <int NT>
+__device__ __forceinline__ void last_stage_end(unsigned long long cbest, DevTime* tm, const Geom& g,
+                                               const Phys& ph, unsigned ctas) {
+    __shared__ unsigned long long wmax[NT / 32];
+    __shared__ int last;
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, cbest, o);
+        cbest = x > cbest ? x : cbest;
+    }
+    if ((t & 31) == 0) wmax[t >> 5] = cbest;
+    __syncthreads();
+    if (t == 0) {
+        unsigned long long m = wmax[0];
+        for (int w = 1; w < NT / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
+        atomicMax(&tm->cmax_acc, m);
+        __threadfence();
+        last = atomicAdd(&tm->done_ctas, 1u) == ctas - 1;
+    }
+    __syncthreads();
+    if (last && t == 0) {
+        __threadfence();
+        step_epilogue(tm, g, ph, 1);
+    }
+}
+
 // ------------------------------------------------------------ x-y plane stage
 // THREE = false: out = c1*uc - c2*dF (stage 1); true: out = c1*u0 + c2*uc -
 // c3*dF.  out never aliases uc (neighbours of uc are read while out is
@@ -370,28 +399,114 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
         Pm1 = P0;
         P0 = P1;
     }
-    if (LAST) {
-        __shared__ unsigned long long wmax[NT / 32];
-        __shared__ int last;
+    if (LAST) last_stage_end<NT>(cbest, tm, g, ph, gridDim.x * gridDim.y * gridDim.z);
+}
+
+// ------------------------------------------------------------ long 1D rows
+// One RK stage of a 1D run in one launch: the x part of k_stage3d on one row,
+// each CTA of 128 threads updating 124 cells, with the x sides' ghost fill in
+// the CTAs that hold ghosts (they also write them back: a frame's ghost strips
+// come from there).  KIND 0: out = c1*uc - c2*dF; 1: out = c1*u0 + c2*uc -
+// c3*dF; 2: as 1, the step's last stage (CFL reduction and epilogue); 3: with
+// the second half kick too.  The expressions are the per-phase kernels'
+// (k_c2p, k_flux, k_update, k_kick, k_cfl), so the bits are the same; those
+// took 11 launches per RK2 step and converted every ghost row of the array
+// (262143 cells, parity: 90 us per step; FP64 alone needs 9).
+constexpr int kRowThreads = 128;
+template <int KIND, bool PLM>
+__global__ void __launch_bounds__(kRowThreads, kStage3dThreadsPerSM / kRowThreads)
+    k_row_stage(double* uc, const double* u0, double* out, Geom g, Phys ph, double c1, double c2,
+                double c3, DevTime* tm, int has_z, int tiles) {
+    if (!tm->active) return;
+    constexpr int NT = kRowThreads;
+    constexpr bool THREE = KIND >= 1, LAST = KIND >= 2;
+    __shared__ double sP[5][NT];
+    __shared__ double sXL[5][NT];
+    __shared__ double sF[5][NT];
+    const int t = threadIdx.x;
+    const int tl = t > 0 ? t - 1 : 0;
+    const int tr = t < NT - 1 ? t + 1 : t;
+    const double dtdx = tm->dt * g.dxRec;
+    // raw state and base state of this thread's cell of a tile, ghosts filled
+    auto load = [&](int tile, Q5& q, double (&b0)[5]) {
+        const int xi = g.ib - 2 + tile * (NT - 4) + t;
+        if (xi < g.ib || (xi >= g.ie && xi < g.lenx))
+            bc_fill_one(uc, g, ph, 0, xi >= g.ie, xi < g.ib ? xi : xi - g.ie);
+        const long long c = sidx(g, g.kb, g.jb, xi < g.lenx ? xi : g.lenx - 1);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long x = __shfl_xor_sync(0xffffffffu, cbest, o);
-            cbest = x > cbest ? x : cbest;
+        for (int v = 0; v < 5; ++v) {
+            q.q[v] = uc[v * g.vstride + c];
+            if (THREE) b0[v] = u0[v * g.vstride + c];
         }
-        if ((t & 31) == 0) wmax[t >> 5] = cbest;
+    };
+    Q5 qn;
+    double bn[5];
+    load(blockIdx.x, qn, bn);
+    unsigned long long cbest = 0ull;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int xi = g.ib - 2 + tile * (NT - 4) + t;
+        const bool do_cell = t >= 2 && t <= NT - 3 && xi < g.ie;
+        const Q5 q = qn;
+        double b0[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) b0[v] = bn[v];
+        if (tile + (int)gridDim.x < tiles) load(tile + gridDim.x, qn, bn);  // arrives meanwhile
+        const W5 P = c2p_q(q, ph);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) sP[v][t] = P.v[v];
         __syncthreads();
-        if (t == 0) {
-            unsigned long long m = wmax[0];
-            for (int w = 1; w < NT / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
-            atomicMax(&tm->cmax_acc, m);
-            __threadfence();
-            const unsigned total = gridDim.x * gridDim.y * gridDim.z;
-            last = atomicAdd(&tm->done_ctas, 1u) == total - 1;
+        double xr[5];
+        if (PLM) {
+            double a[5], d[5], h[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+                a[v] = sP[v][tl];
+                d[v] = sP[v][tr];
+            }
+            half_slopes5(a, P.v, d, h);
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+                sXL[v][t] = P.v[v] + h[v];
+                xr[v] = P.v[v] - h[v];
+            }
+        } else {
+#pragma unroll
+            for (int v = 0; v < 5; ++v) sXL[v][t] = xr[v] = P.v[v];
         }
         __syncthreads();
-        if (last && t == 0) {
-            __threadfence();
-            step_epilogue(tm, g, ph, 1);
+        Flux5 f;
+        hllc<true, kSel>(sXL[gk::P_RHO][tl], sXL[gk::P_VX][tl], sXL[gk::P_VY][tl],
+                         sXL[gk::P_VZ][tl], sXL[gk::P_PRE][tl], xr[gk::P_RHO], xr[gk::P_VX],
+                         xr[gk::P_VY], xr[gk::P_VZ], xr[gk::P_PRE], ph, f);
+        double fx[5];
+        fx[gk::S_DEN] = f.d;
+        fx[gk::S_MTX] = f.n;
+        fx[gk::S_MTY] = f.t1;
+        fx[gk::S_MTZ] = f.t2;
+        fx[gk::S_ENG] = f.e;
+#pragma unroll
+        for (int v = 0; v < 5; ++v) sF[v][t] = fx[v];
+        __syncthreads();
+        if (do_cell) {
+            double r[5];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+                const double dF = (sF[v][tr] - fx[v]) * dtdx;
+                if (THREE) r[v] = c1 * b0[v] + c2 * q.q[v] - c3 * dF;
+                else r[v] = c1 * q.q[v] - c2 * dF;
+            }
+            floors5(r, ph, tm);
+            if (LAST) {
+                if (KIND == 3) kick_cell<false>(r, g, ph, tm->dt, tm->t, 1, xi, g.jb, g.kb);
+                const unsigned long long b = (unsigned long long)__double_as_longlong(
+                    cell_cmax(r[gk::S_DEN], r[gk::S_MTX], r[gk::S_MTY], r[gk::S_MTZ], r[gk::S_ENG], ph,
+                              has_z));
+                cbest = b > cbest ? b : cbest;
+            }
+            const long long c = sidx(g, g.kb, g.jb, xi);
+#pragma unroll
+            for (int v = 0; v < 5; ++v) out[v * g.vstride + c] = r[v];
         }
     }
+    if (LAST) last_stage_end<NT>(cbest, tm, g, ph, gridDim.x);
 }
