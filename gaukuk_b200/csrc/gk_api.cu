@@ -403,7 +403,7 @@ int stage_rows(const gk::Geom& g, int threads, bool parity) {
 // at every face (TMA rows; unless gk_set_flux_model_fused turned that off).
 // Path 2, the 3D stage (z fluxes, then one fused x-y stage per plane),
 // applies to 3D RK2/RK3 runs (forward Euler updates in place, which the
-// fused stage cannot).  Path 3, a 1D run in one CTA (k_run1d, many steps
+// fused stage cannot).  Path 3, a 1D run in one CTA or cluster (k_run1d, many steps
 // per launch), applies to 1D runs of up to 1024 cells per row (lenx) with
 // the device's own ghost fills (copy, periodic, reflecting, outflow) and no
 // source term, learned correction or host routine.  Path 0 is generic.

@@ -1,6 +1,7 @@
 """The 1D row stage (path 0): against the oracle at the edges of its tiles (124
-cells, one tile per CTA up to 444 of them) and against the one-CTA path, whole
-frames with their ghosts, on every pair of x sides."""
+cells, one tile per CTA up to 444 of them) and against the path of short rows
+(path 3, in one CTA or a cluster), whole frames with their ghosts, on every pair
+of x sides."""
 import numpy as np
 import pytest
 
@@ -40,9 +41,11 @@ def test_rows_equal_the_oracle(nx, grav, integrator):
 
 @pytest.mark.parametrize("left", [0, 1, 2, 3])
 @pytest.mark.parametrize("right", [0, 1, 2, 3])
-def test_rows_equal_the_one_cta_path(left, right, monkeypatch):
+def test_rows_equal_the_short_row_path(left, right, monkeypatch):
     from gaukuk_b200.sim import Sim
-    for nx, integrator, rc_order in ((248, 2, 2), (300, 3, 1)):
+    # one CTA up to 316 cells, then 3 to 8 CTAs in a cluster
+    for nx, integrator, rc_order in ((2, 2, 2), (3, 3, 2), (248, 2, 2), (316, 3, 1), (317, 2, 2), (385, 1, 2),
+                                     (640, 3, 2), (1020, 2, 2), (1020, 3, 1)):
         p, c = _problem(nx, (left, right), integrator, rc_order)
         out = []
         for run1d in ("1", "0"):
