@@ -396,6 +396,36 @@ int stage_rows(const gk::Geom& g, int threads, bool parity) {
     return (int)std::max(12LL, std::min(24LL, (tiles + 4 * slots - 1) / (4 * slots)));
 }
 
+// Whether a small grid runs the fused 2D stage in tiles of 28 columns x 4 or 10
+// rows (k_stage2d_tile) instead of the marching kernels: the rows, or 0.  A
+// tile's CTA takes one row time per tile it is given (two of 4 rows or one of 10
+// are resident per SM), the marching CTA a prologue and a row time per row, more
+// so the more CTAs share its SM.  Model of an RK2 step (us), fitted to the
+// measurements in brackets (parity / fast, KH, marching -> tiles):
+//   tiles of 4, one per CTA: 11.1 / 9.2 [64^2: 17.2 -> 10.9 / 13.4 -> 8.9];
+//   tiles of 10, n per CTA: 6.6 + 6.5 n / 6.4 + 4.05 n [192^2: 19.2 -> 13.3 /
+//   14.3 -> 10.6; 256^2: 22.7 -> 19.7 / 16.1 -> 14.6; 384^2: 33.8 -> 32.3 / 22.7 ->
+//   22.5];
+//   marching, one wave of r rows filling a share L of the slots: 3 + (r + 1.4)
+//   (4.2 + 2.1 L) / 3 + (r + 1.4)(2.9 + 2.0 L) [512^2, r = 6 / 4: 45.3 / 27.9].
+// Tiles are taken where they save at least 9 % by it, so that a grid whose tiles
+// are partly empty does not lose (1000x60: 19.5 / 14.6 either way).
+// GK_STAGE_TILE overrides (tuning).
+int stage_tile_rows(const gk::Geom& g, int threads, int rows, bool parity) {
+    const int forced = env_int("GK_STAGE_TILE", -1);
+    if (forced >= 0) return forced == 4 || forced == 10 ? forced : 0;
+    if (env_int("GK_STAGE_ROWS", 0) > 0 || env_int("GK_STAGE_THREADS", 0) > 0) return 0;
+    const long long strips = (g.nx + 27) / 28, slots = 148LL * gk::stage_ctas(threads, parity);
+    const long long march = (long long)((g.nx + threads - 5) / (threads - 4)) * ((g.ny + rows - 1) / rows);
+    if (march > slots) return 0;
+    const double load = (double)march / (double)slots;
+    const double t_march = 3.0 + (rows + 1.4) * (parity ? 4.2 + 2.1 * load : 2.9 + 2.0 * load);
+    if (strips * ((g.ny + 3) / 4) <= 2 * 148) return 4;
+    const long long n = (strips * ((g.ny + 9) / 10) + 147) / 148;
+    const double t_tile = parity ? 6.6 + 6.5 * (double)n : 6.4 + 4.05 * (double)n;
+    return t_tile < 0.91 * t_march ? 10 : 0;
+}
+
 // Path 1, the fused 2D stage, applies to 2D RK2/RK3 runs with MTZ
 // identically zero, no z gravity (it would make MTZ non-zero) and no point
 // masses (their kicks run between the fused stages' CFL reduction and the
@@ -979,7 +1009,9 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
         h->ctx.stage_threads = stage_threads_for(g);
         h->ctx.h2d_rows = stage_rows(g, h->ctx.stage_threads, h->ks == &kParity);
         h->ctx.learn_rows = learn_stage_rows(g, h->ctx.stage_threads);
+        h->ctx.tile_rows = stage_tile_rows(g, h->ctx.stage_threads, h->ctx.h2d_rows, h->ks == &kParity);
     } else {
+        h->ctx.tile_rows = 0;
         h->ctx.h2d_rows = h->tiling_rows;
         h->ctx.learn_rows = 0;
     }
@@ -1359,6 +1391,8 @@ int gk_internal_build_ctx(const gk_grid_desc* gd, const gk_phys_desc* pd, gk::Ct
     tmp.ctx.use_tma = env_int("GK_STAGE_TMA", 1) != 0;
     tmp.ctx.stage_threads = stage_threads_for(tmp.ctx.g);
     tmp.ctx.h2d_rows = stage_rows(tmp.ctx.g, tmp.ctx.stage_threads, pd->mode != GK_MODE_FAST);
+    tmp.ctx.tile_rows = stage_tile_rows(tmp.ctx.g, tmp.ctx.stage_threads, tmp.ctx.h2d_rows,
+                                        pd->mode != GK_MODE_FAST);
     *ctx = tmp.ctx;
     return GK_OK;
 }
@@ -1371,6 +1405,7 @@ extern "C" int gk_set_tiling(gk_handle* h, int threads, int rows) {
     if (rows < 1) return fail(h, GK_ERR_INVALID, "rows per segment must be positive");
     h->ctx.stage_threads = threads;
     h->ctx.h2d_rows = rows;
+    h->ctx.tile_rows = 0;
     h->ctx.learn_rows = 0;  // forced rows serve both stages
     h->tiling_set = true;
     h->tiling_rows = rows;

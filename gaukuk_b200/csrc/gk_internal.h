@@ -132,6 +132,8 @@ struct Ctx {
     Phys ph;
     DevTime* tm;
     int has_vz;      // 2D: MTZ not identically zero -> generic path
+    int tile_rows;      // fused 2D stage in tiles of 28 columns x this many rows (4 or
+                        // 10; small grids), or 0: the marching kernels below
     int h2d_rows;       // fused 2D kernel: rows per CTA segment
     int use_tma;        // fused 2D kernel: rows staged in shared memory by TMA
     int stage_threads;  // fused 2D kernel (TMA): threads per CTA, 64 / 128 / 256

@@ -1245,7 +1245,185 @@ __global__ void __launch_bounds__(kStageThreads, 3)
     }
 }
 
+// The end of a step's last stage: the CTA's largest CFL speed (bit pattern)
+// into the clock; the last of `ctas` CTAs runs the step epilogue (a slab of a
+// split grid leaves that to launch_epilogue, after the maximum over all slabs).
+template <int NT>
+__device__ __forceinline__ void last_stage_end(unsigned long long cbest, DevTime* tm, const Geom& g,
+                                               const Phys& ph, unsigned ctas) {
+    __shared__ unsigned long long wmax[NT / 32];
+    __shared__ int last;
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, cbest, o);
+        cbest = x > cbest ? x : cbest;
+    }
+    if ((t & 31) == 0) wmax[t >> 5] = cbest;
+    __syncthreads();
+    if (t == 0) {
+        unsigned long long m = wmax[0];
+        for (int w = 1; w < NT / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
+        atomicMax(&tm->cmax_acc, m);
+        last = 0;
+        if (!ph.defer_epilogue) {
+            __threadfence();
+            last = atomicAdd(&tm->done_ctas, 1u) == ctas - 1;
+        }
+    }
+    __syncthreads();
+    if (last && t == 0) {
+        __threadfence();
+        step_epilogue(tm, g, ph, 1);
+    }
+}
 
+// ------------------------------------------------------------ fused 2D stage, small grids
+// The same stage for grids that leave the marching kernel's tiles only a few
+// rows: those cost a prologue of about 1.3 row times and a row time per row, one
+// after the other, each a dependency chain of about 2 us in parity mode.  Here a
+// CTA updates a tile of 28 columns x TY rows in one row time: warp w holds row
+// y0 - 1 + w (two columns of halo on each side), the outer two warps convert the
+// rows beyond theirs too, and row exchanges along y go through shared memory
+// (three barriers), along x inside the warp.
+template <int TY>
+struct TileShared {
+    double2 w[2][TY + 4][32];   // primitives of rows y0-2 .. y0+TY+1
+    double2 up[2][TY + 2][32];  // upper y states of rows y0-1 .. (index w)
+    double2 xl[2][TY + 2][32];  // right x states, then x fluxes
+    double2 fy[2][TY + 2][32];  // flux of each row's lower y face
+};
+constexpr int tile_ctas(int ty) { return gk::stage_ctas(64, !GK_FASTMATH) * 64 / (32 * (ty + 2)); }
+template <int TY, int KIND, bool PLM>
+__global__ void __launch_bounds__(32 * (TY + 2), tile_ctas(TY))
+    k_stage2d_tile(const double* __restrict__ uc, const double* u0, double* out, Geom g, Phys ph,
+                   double c1, double c2, double c3, DevTime* tm, int tx) {
+    constexpr bool THREE = KIND >= 1;
+    constexpr bool LAST = KIND == 2;
+    if (!tm->active) return;
+    extern __shared__ __align__(16) unsigned char dynt[];
+    auto& sm = *reinterpret_cast<TileShared<TY>*>(dynt);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long vs = g.vstride, P = g.pitch;
+    const bool inner = w >= 1 && w <= TY;  // a row of the tile
+    // column, row and offset of this thread's cell in a tile; columns and rows
+    // past the array are clamped into it (they feed no cell of the grid)
+    const int tiles = tx * ((g.ny + TY - 1) / TY);
+    auto col = [&](int tile) { return g.ib - 2 + tile % tx * 28 + lane; };
+    auto row = [&](int tile) { return g.jb + tile / tx * TY - 1 + w; };
+    auto at = [&](int xi, int j) {
+        return sidx(g, g.kb, j < g.leny ? j : g.leny - 1, xi < g.lenx ? xi : g.lenx - 1);
+    };
+    // loads of the row, of the row beyond it (outer warps) and of the base state
+    Q4 qn, qbn{1, 0, 0, 1}, b0n{0, 0, 0, 0};
+    auto load = [&](int tile) {
+        const int xi = col(tile), y = row(tile);
+        qn = ldq(uc, vs, at(xi, y));
+        if (!inner) qbn = ldq(uc, vs, at(xi, w == 0 ? y - 1 : y + 1));
+        if (THREE && inner) {
+            const long long c = at(xi, y);
+            b0n = Q4{u0[c], u0[vs + c], u0[2 * vs + c], u0[3 * vs + c]};
+        }
+    };
+    auto put = [&](double2(*s)[32], int stride, const W4& a) {  // rows of one exchange array
+        s[0][lane] = make_double2(a.r, a.vx);
+        s[stride][lane] = make_double2(a.vy, a.p);
+    };
+    auto get = [&](const double2(*s)[32], int stride, int l) {
+        const double2 a = s[0][l], b = s[stride][l];
+        return W4{a.x, a.y, b.x, b.y};
+    };
+    const double dt = tm->dt;
+    const double dtdx = dt * g.dxRec, dtdy = dt * g.dyRec;
+    unsigned long long cbest = 0ull;
+    load(blockIdx.x);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int xi = col(tile), y = row(tile);
+        const bool do_cell = inner && lane >= 2 && lane < 30 && xi < g.ie && y < g.je;
+        const Q4 q = qn, qb = qbn, b0 = b0n;
+        if (tile + (int)gridDim.x < tiles) load(tile + gridDim.x);  // arrives meanwhile
+        const W4 Pc = c2p4(q, ph);
+        put(&sm.w[0][w + 1], TY + 4, Pc);
+        if (!inner) put(&sm.w[0][w == 0 ? 0 : TY + 3], TY + 4, c2p4(qb, ph));
+        __syncthreads();
+        const int ll = lane > 0 ? lane - 1 : 0, lr = lane < 31 ? lane + 1 : 31;
+        W4 xr = Pc, lo = Pc, up = Pc, xl = Pc;
+        if (PLM) {
+            SlopeRange rg;
+            clear(rg);
+            const W4 below = get(&sm.w[0][w], TY + 4, lane), above = get(&sm.w[0][w + 2], TY + 4, lane);
+            const W4 lft = get(&sm.w[0][w + 1], TY + 4, ll), rgt = get(&sm.w[0][w + 1], TY + 4, lr);
+            W4 sy = vl4(below, Pc, above, rg);
+            W4 sx = vl4(lft, Pc, rgt, rg);
+#if !GK_FASTMATH
+            if (out_of_range(rg)) {
+                sy = vl4_any(below, Pc, above);
+                sx = vl4_any(lft, Pc, rgt);
+            }
+#endif
+            lo = minus_half(Pc, sy);
+            up = plus_half(Pc, sy);
+            xr = minus_half(Pc, sx);
+            xl = plus_half(Pc, sx);
+        }
+        put(&sm.up[0][w], TY + 2, up);
+        put(&sm.xl[0][w], TY + 2, xl);
+        __syncthreads();
+        Flux5 fx{}, fy{};
+        if (w >= 1) {  // row y0 - 1 has no face of the tile
+            const W4 xls = get(&sm.xl[0][w], TY + 2, ll);
+            const W4 yl = get(&sm.up[0][w - 1], TY + 2, lane);
+            hllc_xy(xls, xr, fx, yl, lo, fy, ph);
+            __syncwarp();  // xl of the row is read
+            put(&sm.xl[0][w], TY + 2, W4{fx.d, fx.n, fx.t1, fx.e});
+            put(&sm.fy[0][w], TY + 2, W4{fy.d, fy.n, fy.t1, fy.e});
+        }
+        __syncthreads();
+        if (do_cell) {
+            const W4 fr = get(&sm.xl[0][w], TY + 2, lr), fu = get(&sm.fy[0][w + 1], TY + 2, lane);
+            const double dF0 = (fr.r - fx.d) * dtdx + (fu.r - fy.d) * dtdy;
+            const double dF1 = (fr.vx - fx.n) * dtdx + (fu.vy - fy.t1) * dtdy;
+            const double dF2 = (fr.vy - fx.t1) * dtdx + (fu.vx - fy.n) * dtdy;
+            const double dF3 = (fr.p - fx.e) * dtdx + (fu.p - fy.e) * dtdy;
+            double r[4];
+            if (THREE) {
+                r[0] = c1 * b0.d + c2 * q.d - c3 * dF0;
+                r[1] = c1 * b0.mx + c2 * q.mx - c3 * dF1;
+                r[2] = c1 * b0.my + c2 * q.my - c3 * dF2;
+                r[3] = c1 * b0.e + c2 * q.e - c3 * dF3;
+            } else {
+                r[0] = c1 * q.d - c2 * dF0;
+                r[1] = c1 * q.mx - c2 * dF1;
+                r[2] = c1 * q.my - c2 * dF2;
+                r[3] = c1 * q.e - c2 * dF3;
+            }
+            const double invk = floors4_inv(r, ph, tm);
+            if (LAST) {
+                if (ph.has_grav) {
+                    const double hdt = 0.5 * dt;
+                    if (ph.grav[0] != 0) {
+                        r[3] += r[1] * ph.grav[0] * hdt;
+                        r[1] += r[0] * ph.grav[0] * hdt;
+                    }
+                    if (ph.grav[1] != 0) {
+                        r[3] += r[2] * ph.grav[1] * hdt;
+                        r[2] += r[0] * ph.grav[1] * hdt;
+                    }
+                }
+                const unsigned long long b =
+                    (unsigned long long)__double_as_longlong(cell_cmax_inv(r[1], r[2], r[3], invk, ph));
+                cbest = b > cbest ? b : cbest;
+            }
+            const long long oc = at(xi, GK_CHK(y, g.jb, g.je, 7));
+            out[oc] = r[0];
+            out[vs + oc] = r[1];
+            out[2 * vs + oc] = r[2];
+            out[3 * vs + oc] = r[3];
+            if (ph.periodic_images) store_images(out, vs, P, oc, xi, y, g, r);
+        }
+    }
+    if (LAST) last_stage_end<32 * (TY + 2)>(cbest, tm, g, ph, gridDim.x);
+}
 
 // ------------------------------------------------------------ fused 2D stage, TMA rows
 // The same stage with its input rows staged in shared memory by the tensor
@@ -2144,9 +2322,39 @@ void launch_stage2d_learn(const Ctx& c, const double* uc, const double* u0, doub
     else launch_stage2d_learn_nt<128>(c, mc, m0, out, kind, c1, c2, c3, model, gate, fired, s);
 }
 
+template <int TY, int KIND, bool PLM>
+static void launch_stage2d_tile_k(const Ctx& c, const double* uc, const double* u0, double* out,
+                                  double c1, double c2, double c3, cudaStream_t s) {
+    const Geom& g = c.g;
+    constexpr int bytes = (int)sizeof(TileShared<TY>);
+    static std::atomic<unsigned long long> attr_set{0};
+    if (gk::first_on_device(attr_set))
+        cudaFuncSetAttribute(k_stage2d_tile<TY, KIND, PLM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const int tx = (g.nx + 27) / 28, tiles = tx * ((g.ny + TY - 1) / TY);
+    const int grid = min(tiles, 148 * tile_ctas(TY));
+    k_stage2d_tile<TY, KIND, PLM><<<grid, 32 * (TY + 2), bytes, s>>>(uc, u0, out, g, c.ph, c1, c2, c3, c.tm, tx);
+}
+template <int TY>
+static void launch_stage2d_tile(const Ctx& c, const double* uc, const double* u0, double* out, int kind,
+                                double c1, double c2, double c3, cudaStream_t s) {
+#define GK_TILE(K, PL) launch_stage2d_tile_k<TY, K, PL>(c, uc, u0, out, c1, c2, c3, s)
+    if (c.ph.plm) {
+        if (kind == 0) GK_TILE(0, true);
+        else if (kind == 1) GK_TILE(1, true);
+        else GK_TILE(2, true);
+    } else {
+        if (kind == 0) GK_TILE(0, false);
+        else if (kind == 1) GK_TILE(1, false);
+        else GK_TILE(2, false);
+    }
+#undef GK_TILE
+}
+
 void launch_stage2d(const Ctx& c, const double* uc, const double* u0, double* out, int kind,
                     double c1, double c2, double c3, cudaStream_t s) {
     const Geom& g = c.g;
+    if (c.tile_rows == 4) return launch_stage2d_tile<4>(c, uc, u0, out, kind, c1, c2, c3, s);
+    if (c.tile_rows == 10) return launch_stage2d_tile<10>(c, uc, u0, out, kind, c1, c2, c3, s);
     const int rows = c.h2d_rows;
     if (c.use_tma) {
         const int nt = c.stage_threads;

@@ -199,35 +199,6 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-// The end of a step's last stage: the CTA's largest CFL speed (bit pattern)
-// into the clock; the last of `ctas` CTAs runs the step epilogue.
-template <int NT>
-__device__ __forceinline__ void last_stage_end(unsigned long long cbest, DevTime* tm, const Geom& g,
-                                               const Phys& ph, unsigned ctas) {
-    __shared__ unsigned long long wmax[NT / 32];
-    __shared__ int last;
-    const int t = threadIdx.x;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long x = __shfl_xor_sync(0xffffffffu, cbest, o);
-        cbest = x > cbest ? x : cbest;
-    }
-    if ((t & 31) == 0) wmax[t >> 5] = cbest;
-    __syncthreads();
-    if (t == 0) {
-        unsigned long long m = wmax[0];
-        for (int w = 1; w < NT / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
-        atomicMax(&tm->cmax_acc, m);
-        __threadfence();
-        last = atomicAdd(&tm->done_ctas, 1u) == ctas - 1;
-    }
-    __syncthreads();
-    if (last && t == 0) {
-        __threadfence();
-        step_epilogue(tm, g, ph, 1);
-    }
-}
-
 // ------------------------------------------------------------ x-y plane stage
 // THREE = false: out = c1*uc - c2*dF (stage 1); true: out = c1*u0 + c2*uc -
 // c3*dF.  out never aliases uc (neighbours of uc are read while out is
