@@ -248,6 +248,9 @@ static const char* const kClassNames[K_NCLASS] = {
                               const float* model, const gk::FluxGate& gate, unsigned* fired,   \
                               cudaStream_t s);                                                 \
     void launch_begin(const gk::Ctx& c, double dtoutput, int steps, cudaStream_t s);           \
+    void launch_noalloc_begin(const gk::Ctx& c, const double* u, double dtmax, int* flag_acc,  \
+                              int* flag, unsigned long long* ticket_out,                       \
+                              unsigned long long ticket, cudaStream_t s);                      \
     void launch_epilogue(const gk::Ctx& c, cudaStream_t s);                                    \
     int checked_report(unsigned long long* count, unsigned long long* first);                  \
     void launch_mtz_check(const gk::Ctx& c, const double* u, int* flag, cudaStream_t s);       \

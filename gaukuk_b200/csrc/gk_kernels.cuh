@@ -691,6 +691,65 @@ __global__ void k_begin(DevTime* tm, Geom g, Phys ph, double dtoutput, int steps
     begin_one(tm, g, ph, dtoutput, steps);
 }
 
+// Start of a step on a caller-owned 2D state (gk_noalloc.cu) in one pass: the
+// check that MTZ is zero on every active cell (k_mtz_check), CalCmax (k_cfl),
+// and in the last CTA the clock of one step from t = 0 with dtUntilOutput =
+// dtmax (begin_one); with a non-zero MTZ the run stays inactive.  A reset, the
+// check with a copy to the host, the reduction and the begin kernel took 26 us
+// of a 130 x 94 step's 92.
+__global__ void __launch_bounds__(256)
+    k_noalloc_begin(const double* __restrict__ u, Geom g, Phys ph, DevTime* tm, double dtmax,
+                    int* flag_acc, int* flag, unsigned long long* ticket_out,
+                    unsigned long long ticket) {
+    unsigned long long best = 0ull;
+    int mtz = 0;
+    for (int j = g.jb + blockIdx.y; j < g.je; j += gridDim.y) {
+        const int i = g.ib + blockIdx.x * blockDim.x + threadIdx.x;
+        if (i >= g.ie) continue;
+        const long long c = sidx(g, g.kb, j, i);
+        const double mz = u[gk::S_MTZ * g.vstride + c];
+        mtz |= mz != 0.0;
+        const unsigned long long b = (unsigned long long)__double_as_longlong(
+            cell_cmax(u[gk::S_DEN * g.vstride + c], u[gk::S_MTX * g.vstride + c],
+                      u[gk::S_MTY * g.vstride + c], mz, u[gk::S_ENG * g.vstride + c], ph, true));
+        best = b > best ? b : best;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, best, o);
+        best = x > best ? x : best;
+    }
+    __shared__ unsigned long long wmax[8];
+    __shared__ bool last;
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = best;
+    mtz = __syncthreads_or(mtz);
+    if (threadIdx.x == 0) {
+        unsigned long long m = wmax[0];
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = wmax[w] > m ? wmax[w] : m;
+        atomicMax(&tm->cmax_acc, m);
+        if (mtz) atomicOr(flag_acc, 1);
+        __threadfence();
+        last = atomicAdd(&tm->done_ctas, 1u) == gridDim.x * gridDim.y - 1;
+    }
+    __syncthreads();
+    if (!last || threadIdx.x != 0) return;
+    __threadfence();
+    const unsigned long long seed = (unsigned long long)__double_as_longlong(1e-16);
+    const unsigned long long acc = atomicAdd(&tm->cmax_acc, 0ull);
+    const int bad = atomicExch(flag_acc, 0);
+    DevTime t{};
+    t.cmax_last = __longlong_as_double((long long)(acc > seed ? acc : seed));
+    t.dt = 1e10;
+    t.cmax_acc = seed;
+    t.is_continue = 1;
+    t.status = t.cmax_last <= DBL_MAX ? 0 : gk::STATUS_NONFINITE;
+    begin_one(&t, g, ph, dtmax, 0);
+    if (bad) t.active = 0;
+    *tm = t;
+    *flag = bad;
+    *ticket_out = ticket;
+}
+
 // The step epilogue of a slab whose last stage deferred it: cmax_acc holds
 // the maximum over every slab of the grid by now.
 __global__ void k_epilogue(DevTime* tm, Geom g, Phys ph) {
@@ -2422,6 +2481,13 @@ void launch_ens_bc(const gk::EnsInst* inst, int n, int which, int max_count, cud
 
 void launch_ens_begin(const gk::EnsInst* inst, int n, double dtoutput, int steps, cudaStream_t s) {
     k_ens_begin<<<(n + 63) / 64, 64, 0, s>>>(inst, n, dtoutput, steps);
+}
+
+void launch_noalloc_begin(const Ctx& c, const double* u, double dtmax, int* flag_acc, int* flag,
+                          unsigned long long* ticket_out, unsigned long long ticket, cudaStream_t s) {
+    const unsigned bx = (c.g.nx + 255) / 256;
+    const dim3 grid(bx, min((unsigned)c.g.ny, 148u * 8u / bx + 1u));
+    k_noalloc_begin<<<grid, 256, 0, s>>>(u, c.g, c.ph, c.tm, dtmax, flag_acc, flag, ticket_out, ticket);
 }
 
 void launch_epilogue(const Ctx& c, cudaStream_t s) { k_epilogue<<<1, 1, 0, s>>>(c.tm, c.g, c.ph); }

@@ -20,7 +20,6 @@
 // 5 * vstride doubles fit (about 1290 x 1290 cells).
 #include <atomic>
 #include <cstdio>
-#include <cstring>
 #include <string>
 
 #include "gaukuk_cuda.h"
@@ -35,13 +34,17 @@ constexpr long long kScratchDoubles = 1LL << 23;  // 64 MiB
 constexpr int kMaxDevices = 64;
 
 // Scratch: the intermediate RK stage state (5 variable planes in the device
-// layout), then the device clock, the MTZ check flag and the ticket of the
-// call whose clock reset ran last.
+// layout), then what a call reads back: the device clock, whether MTZ was
+// non-zero, and the ticket of the call whose clock was set last.
+struct NoallocResult {
+    gk::DevTime clock;
+    unsigned long long ticket;
+    int flag;
+    int flag_acc;  // the running check of one call; zero between calls
+};
 struct NoallocScratch {
     double stage[kScratchDoubles];
-    gk::DevTime clock;
-    int flag;
-    unsigned long long ticket;
+    NoallocResult res;
 };
 
 static __device__ __align__(256) NoallocScratch gk_noalloc_scratch;
@@ -51,36 +54,11 @@ static __device__ __align__(256) NoallocScratch gk_noalloc_scratch;
 // at the same time each look it up and store the same value.
 std::atomic<NoallocScratch*> g_scratch_addr[kMaxDevices];
 
-// Call tickets: the reset kernel stores its call's ticket, so a call that
+// Call tickets: the begin kernel stores its call's ticket, so a call that
 // finds its own ticket and step 1 in the clock knows that its launches ran
 // (without reading cudaGetLastError, which would also report errors left by
 // unrelated work).
 std::atomic<unsigned long long> g_ticket{0};
-
-// Resets the clock for one step starting at time 0 with no output limit.
-__global__ void k_noalloc_reset(gk::DevTime* tm, int* flag, unsigned long long* ticket_out,
-                                unsigned long long ticket) {
-    gk::DevTime t{};
-    t.t = 0;
-    t.dt = 1e10;
-    t.tNext = 0;
-    t.dtUntilOutput = 1e10;
-    t.cmax_last = 1e-16;
-    double seed = 1e-16;
-    memcpy(&t.cmax_acc, &seed, sizeof(double));
-    t.done_ctas = 0;
-    t.step = 0;
-    t.is_continue = 1;
-    t.active = 1;
-    t.status = 0;
-    t.steps_left = -1;
-    t.nlog = 0;
-    t.log_cap = 0;
-    t.log = nullptr;
-    *tm = t;
-    *flag = 0;
-    *ticket_out = ticket;
-}
 
 }  // namespace
 
@@ -127,47 +105,42 @@ extern "C" int gk_rk2_step_noalloc(const gk_grid_desc* grid, const gk_phys_desc*
     }
     NoallocScratch* sc = g_scratch_addr[dev].load(std::memory_order_acquire);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    c.tm = &sc->clock;
+    c.tm = &sc->res.clock;
     double* stage = sc->stage;
 
     const unsigned long long ticket = ++g_ticket;
-    k_noalloc_reset<<<1, 1, 0, s>>>(&sc->clock, &sc->flag, &sc->ticket, ticket);
     const bool fast = phys->mode == GK_MODE_FAST;
-    auto mtz = fast ? gk_fast::launch_mtz_check : gk_parity::launch_mtz_check;
-    auto cfl = fast ? gk_fast::launch_cfl : gk_parity::launch_cfl;
-    auto begin = fast ? gk_fast::launch_begin : gk_parity::launch_begin;
+    auto begin = fast ? gk_fast::launch_noalloc_begin : gk_parity::launch_noalloc_begin;
     auto bc = fast ? gk_fast::launch_bc : gk_parity::launch_bc;
     auto stage2d = fast ? gk_fast::launch_stage2d : gk_parity::launch_stage2d;
     auto kick = fast ? gk_fast::launch_kick : gk_parity::launch_kick;
-    mtz(c, state, &sc->flag, s);
-    int flag = 0;
-    if (cudaMemcpyAsync(&flag, &sc->flag, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return GK_ERR_CUDA;
-    if (flag) {
-        std::fprintf(stderr, "gk_rk2_step_noalloc: MTZ is not zero; the fused 2D step needs vz = 0\n");
-        return GK_ERR_UNSUPPORTED;
-    }
     // Sim::Advance for one step with dtUntilOutput = dtmax (sim.cpp:77-81):
-    // cmax of the state, dt, the first gravity half kick (sim.cpp:85-86),
-    // then the two RK2 stages; the last stage applies the second half kick
-    // and its epilogue advances the clock.
-    cfl(c, state, 0, s);
-    begin(c, dtmax, 0, s);
+    // one pass over the state checks that MTZ is zero and reduces cmax, and its
+    // last CTA sets the clock with dt (inactive, so that nothing after it
+    // runs, when MTZ is not zero); then the first gravity half kick
+    // (sim.cpp:85-86) and the two RK2 stages; the last stage applies the second
+    // half kick and its epilogue advances the clock.  On a grid periodic on all
+    // sides the first stage writes the stage state's ghosts itself.
+    begin(c, state, dtmax, &sc->res.flag_acc, &sc->res.flag, &sc->res.ticket, ticket, s);
     if (c.ph.has_grav) kick(c, state, 0, s);
     bc(c, state, s);
-    stage2d(c, state, nullptr, stage, 0, 1.0, 1.0, 0.0, s);
-    bc(c, stage, s);
+    gk::Ctx first = c;
+    first.ph.periodic_images = c.ph.bc[0] == 1 && c.ph.bc[1] == 1 && c.ph.bc[2] == 1 && c.ph.bc[3] == 1;
+    stage2d(first, state, nullptr, stage, 0, 1.0, 1.0, 0.0, s);
+    if (!first.ph.periodic_images) bc(c, stage, s);
     stage2d(c, stage, state, state, 2, 0.5, 0.5, 0.5, s);
-    gk::DevTime t{};
-    unsigned long long ran = 0;
-    if (cudaMemcpyAsync(&t, &sc->clock, sizeof(t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(&ran, &sc->ticket, sizeof(ran), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    NoallocResult r{};
+    if (cudaMemcpyAsync(&r, &sc->res, sizeof(r), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return GK_ERR_CUDA;
-    if (ran != ticket) {
+    const gk::DevTime& t = r.clock;
+    if (r.ticket != ticket) {
         std::fprintf(stderr, "gk_rk2_step_noalloc: a kernel of this call did not launch\n");
         return GK_ERR_CUDA;
+    }
+    if (r.flag) {
+        std::fprintf(stderr, "gk_rk2_step_noalloc: MTZ is not zero; the fused 2D step needs vz = 0\n");
+        return GK_ERR_UNSUPPORTED;
     }
     if (t.status & gk::STATUS_TMA_TIMEOUT) {
         std::fprintf(stderr, "gk_rk2_step_noalloc: a TMA row load did not complete within the "
