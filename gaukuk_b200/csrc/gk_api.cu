@@ -1428,7 +1428,7 @@ struct gk_ensemble {
     const KernelSet* ks = nullptr;
     cudaStream_t stream = nullptr;
     gk::EnsInst* dinst = nullptr;
-    int2* dtiles = nullptr;
+    int4* dtiles = nullptr;
     unsigned* dcount = nullptr;  // work counters of the two stages
     int* dany = nullptr;
     int ntiles = 0, max_bc = 0;
@@ -1461,9 +1461,61 @@ __global__ void k_ens_any_active(const gk::EnsInst* __restrict__ inst, int n, in
     if (threadIdx.x == 0) *any = a;
 }
 
+// The tile table: each strip of columns of each instance cut into tiles of the
+// instance's rows, except that the strips of the last, partly filled wave are
+// cut so that it fills the resident CTAs: a tile costs its rows plus about 1.4
+// (its prologue), whether its wave is full or not.  KH instances of 128^2 - 512^2
+// in tiles of 128 threads x 16 rows, fast mode, us per step: 32 instances (4.5
+// waves) 361 -> 352, 21 (3.1 waves) 267 -> 250.
+std::vector<int4> ens_tiles(const gk_ensemble* e, std::vector<int>& per) {
+    struct Strip {
+        int inst, bx, rows;
+    };
+    std::vector<Strip> strips;
+    long long total = 0;
+    for (int i = 0; i < e->n; ++i) {
+        const gk::Geom& g = e->h[i]->ctx.g;
+        const int rows = std::max(1, e->rows[i]);
+        const int tx = (g.nx + e->threads - 5) / (e->threads - 4);
+        for (int bx = 0; bx < tx; ++bx) strips.push_back({i, bx, rows});
+        total += (long long)tx * ((g.ny + rows - 1) / rows);
+    }
+    const long long slots = 148LL * gk::stage_ctas(e->threads, e->ks == &kParity);
+    const long long full = total / slots * slots;  // tiles in full waves
+    long long rest = total, tail_rows = 0;
+    size_t cut = strips.size();  // strips cut .. end belong to the last wave
+    while (rest > full && cut > 0) {
+        const Strip& s = strips[--cut];
+        const int ny = e->h[s.inst]->ctx.g.ny;
+        rest -= (ny + s.rows - 1) / s.rows;
+        tail_rows += ny;
+    }
+    // rows that let the last wave's tiles fit the slots it finds free
+    const long long free_slots = slots + (full - rest);
+    int tail = (int)std::max(2LL, (tail_rows + free_slots - 1) / free_slots);
+    for (;; ++tail) {
+        long long n = 0;
+        for (size_t q = cut; q < strips.size(); ++q) n += (e->h[strips[q].inst]->ctx.g.ny + tail - 1) / tail;
+        if (n <= free_slots || n == (long long)(strips.size() - cut)) break;
+    }
+    std::vector<int4> tiles;
+    per.assign(e->n, 0);
+    for (size_t q = 0; q < strips.size(); ++q) {
+        const Strip& s = strips[q];
+        const gk::Geom& g = e->h[s.inst]->ctx.g;
+        const int rows = q < cut ? s.rows : std::min(s.rows, tail);
+        for (int y = g.jb; y < g.je; y += rows) {
+            tiles.push_back(make_int4(s.inst, s.bx, y, std::min(y + rows, g.je)));
+            ++per[s.inst];
+        }
+    }
+    return tiles;
+}
+
 int ens_build(gk_ensemble* e) {
     std::vector<gk::EnsInst> inst(e->n);
-    std::vector<int2> tiles;
+    std::vector<int> per;
+    const std::vector<int4> tiles = ens_tiles(e, per);
     e->max_bc = 0;
     for (int i = 0; i < e->n; ++i) {
         const gk::Ctx& c = e->h[i]->ctx;
@@ -1476,13 +1528,10 @@ int ens_build(gk_ensemble* e) {
         I.A = e->h[i]->A;
         I.B = e->h[i]->B;
         I.tm = e->h[i]->tm;
-        I.rows = std::max(1, e->rows[i]);
-        I.tiles_x = (g.nx + e->threads - 5) / (e->threads - 4);
-        I.tiles = I.tiles_x * ((g.ny + I.rows - 1) / I.rows);
+        I.tiles = per[i];
         I.g = g;
         I.ph = c.ph;
         I.ph.periodic_images = 0;  // the ensemble fills every instance's ghosts
-        for (int t = 0; t < I.tiles; ++t) tiles.push_back(make_int2(i, t));
         e->max_bc = std::max(e->max_bc, g.ng * std::max(g.nx, g.ny));
     }
     cudaFree(e->dinst);
@@ -1491,10 +1540,10 @@ int ens_build(gk_ensemble* e) {
     e->dtiles = nullptr;
     e->ntiles = (int)tiles.size();
     GK_ECUDA(e, cudaMalloc(&e->dinst, sizeof(gk::EnsInst) * e->n));
-    GK_ECUDA(e, cudaMalloc(&e->dtiles, sizeof(int2) * tiles.size()));
+    GK_ECUDA(e, cudaMalloc(&e->dtiles, sizeof(int4) * tiles.size()));
     GK_ECUDA(e, cudaMemcpy(e->dinst, inst.data(), sizeof(gk::EnsInst) * e->n,
                            cudaMemcpyHostToDevice));
-    GK_ECUDA(e, cudaMemcpy(e->dtiles, tiles.data(), sizeof(int2) * tiles.size(),
+    GK_ECUDA(e, cudaMemcpy(e->dtiles, tiles.data(), sizeof(int4) * tiles.size(),
                            cudaMemcpyHostToDevice));
     if (e->gexec) {
         cudaGraphExecDestroy(e->gexec);

@@ -143,14 +143,14 @@ struct Ctx {
 
 // One instance of an ensemble, as the persistent stage kernel reads it from
 // global memory: tensor maps of its two state buffers, the buffers, its
-// clock, its tiling and geometry.
+// clock, its number of tiles and its geometry.
 struct alignas(64) EnsInst {
     CUtensorMap mapA;
     CUtensorMap mapB;
     double* A;
     double* B;
     DevTime* tm;
-    int rows, tiles_x, tiles;
+    int tiles;  // of this instance
     Geom g;
     Phys ph;
 };
@@ -255,7 +255,7 @@ static const char* const kClassNames[K_NCLASS] = {
     int checked_report(unsigned long long* count, unsigned long long* first);                  \
     void launch_mtz_check(const gk::Ctx& c, const double* u, int* flag, cudaStream_t s);       \
     void launch_ens_stage(int threads, int kind, int plm, const gk::EnsInst* inst,             \
-                          const int2* tiles, int ntiles, unsigned* counter, double c1,          \
+                          const int4* tiles, int ntiles, unsigned* counter, double c1,          \
                           double c2, double c3, cudaStream_t s);                                \
     void launch_ens_bc(const gk::EnsInst* inst, int n, int which, int max_count,               \
                        cudaStream_t s);                                                        \

@@ -1497,7 +1497,7 @@ __global__ void __launch_bounds__(32 * (TY + 2), tile_ctas(TY))
 // only halo lanes.  Waits are bounded: a wait that gives up sets
 // STATUS_TMA_TIMEOUT and the kernel carries on, so it cannot hang.
 //
-// stage_tile_tma does one tile (strip bx, segment by).  The single-problem
+// stage_tile_tma does one tile (strip bx, rows y0 .. y1-1).  The single-problem
 // kernel runs one tile per CTA; the ensemble kernel (k_ens_stage) is
 // persistent: each CTA takes tiles of any instance from a tile table through
 // an atomic counter, reusing its ring and barriers.
@@ -1701,7 +1701,7 @@ template <int NT, int KIND, bool PLM, bool LEARN = false>
 __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CUtensorMap* map0,
                                                double* out, const Geom& g, const Phys& ph,
                                                double c1, double c2, double c3, DevTime* tm,
-                                               int rows, int bx, int by, unsigned tiles_total,
+                                               int bx, int y0, int y1, unsigned tiles_total,
                                                double* ring, double* ring0, StageShared<NT>& sm,
                                                unsigned& seq, unsigned& seq0,
                                                const LearnArgs* la = nullptr) {
@@ -1721,8 +1721,6 @@ __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CU
     const int x0 = g.ib - 2 + bx * COLS;  // box origin column
     const int xi = x0 + t;
     const bool do_cell = t >= 2 && t <= NT - 3 && xi < g.ie;
-    const int y0 = g.jb + by * rows;
-    const int y1 = min(y0 + rows, g.je);
     const int rlo = y0 - 2;
     const long long vs = g.vstride;
     const long long P = g.pitch;
@@ -1805,7 +1803,7 @@ __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CU
             // too, so only the grid's first segment counts its veto
             Flux5 none{};
             const auto st = [&](int) { return stencil_y(Pm2, Pm1, P0, P1); };
-            learn_faces(*la, st, false, false, none, dtdx, do_cell, do_cell && by == 0, fyPrev,
+            learn_faces(*la, st, false, false, none, dtdx, do_cell, do_cell && y0 == g.jb, fyPrev,
                         dtdy, ph, nfired);
             Pm2 = Pm1;
         }
@@ -1989,9 +1987,10 @@ __global__ void __launch_bounds__(NT, gk::stage_ctas(NT, !GK_FASTMATH))
     __shared__ StageShared<NT> sm;
     stage_init_barriers(sm);
     unsigned seq = 0, seq0 = 0;
-    stage_tile_tma<NT, KIND, PLM>(&mapc, &map0, out, g, ph, c1, c2, c3, tm, rows, blockIdx.x,
-                                  blockIdx.y, gridDim.x * gridDim.y, dyn, dyn + kRing * 4 * NT, sm,
-                                  seq, seq0);
+    const int y0 = g.jb + blockIdx.y * rows;
+    stage_tile_tma<NT, KIND, PLM>(&mapc, &map0, out, g, ph, c1, c2, c3, tm, blockIdx.x, y0,
+                                  min(y0 + rows, g.je), gridDim.x * gridDim.y, dyn,
+                                  dyn + kRing * 4 * NT, sm, seq, seq0);
 }
 
 // The fused stage with the learned flux correction at every face.  Dynamic
@@ -2019,17 +2018,18 @@ __global__ void __launch_bounds__(NT, 256 / NT)
     stage_init_barriers(sm);  // its barrier also publishes the weights
     const LearnArgs la{w, lw, gate, fired};
     unsigned seq = 0, seq0 = 0;
-    stage_tile_tma<NT, KIND, PLM, true>(&mapc, &map0, out, g, ph, c1, c2, c3, tm, rows, blockIdx.x,
-                                        blockIdx.y, gridDim.x * gridDim.y, dyn, dyn + kRing * 4 * NT,
-                                        sm, seq, seq0, &la);
+    const int y0 = g.jb + blockIdx.y * rows;
+    stage_tile_tma<NT, KIND, PLM, true>(&mapc, &map0, out, g, ph, c1, c2, c3, tm, blockIdx.x, y0,
+                                        min(y0 + rows, g.je), gridDim.x * gridDim.y, dyn,
+                                        dyn + kRing * 4 * NT, sm, seq, seq0, &la);
 }
 
-// Persistent stage over an ensemble: tiles[i] = (instance, tile of that
-// instance), claimed through *counter (zeroed before the launch).  Stage
+// Persistent stage over an ensemble: tiles[i] = (instance, strip, first row,
+// one past the last row), claimed through *counter (zeroed before the launch).  Stage
 // KIND 0 reads A and writes B; KIND 2 reads B and A and writes A.
 template <int NT, int KIND, bool PLM>
 __global__ void __launch_bounds__(NT, gk::stage_ctas(NT, !GK_FASTMATH))
-    k_ens_stage(const gk::EnsInst* __restrict__ inst, const int2* __restrict__ tiles, int ntiles,
+    k_ens_stage(const gk::EnsInst* __restrict__ inst, const int4* __restrict__ tiles, int ntiles,
                 unsigned* counter, double c1, double c2, double c3) {
     extern __shared__ __align__(128) double dyn[];
     __shared__ StageShared<NT> sm;
@@ -2041,21 +2041,20 @@ __global__ void __launch_bounds__(NT, gk::stage_ctas(NT, !GK_FASTMATH))
         const int id = sm.cur;
         __syncthreads();
         if (id >= ntiles) break;
-        const int2 tl = tiles[id];
+        const int4 tl = tiles[id];
         const gk::EnsInst* I = inst + tl.x;
         DevTime* tm = I->tm;
         if (!tm->active) continue;
         const Geom g = I->g;
         const Phys ph = I->ph;
-        const int bx = tl.y % I->tiles_x, by = tl.y / I->tiles_x;
         if (KIND == 0)
-            stage_tile_tma<NT, KIND, PLM>(&I->mapA, &I->mapA, I->B, g, ph, c1, c2, c3, tm, I->rows,
-                                          bx, by, (unsigned)I->tiles, dyn, dyn + kRing * 4 * NT,
-                                          sm, seq, seq0);
+            stage_tile_tma<NT, KIND, PLM>(&I->mapA, &I->mapA, I->B, g, ph, c1, c2, c3, tm, tl.y, tl.z,
+                                          tl.w, (unsigned)I->tiles, dyn, dyn + kRing * 4 * NT, sm,
+                                          seq, seq0);
         else
-            stage_tile_tma<NT, KIND, PLM>(&I->mapB, &I->mapA, I->A, g, ph, c1, c2, c3, tm, I->rows,
-                                          bx, by, (unsigned)I->tiles, dyn, dyn + kRing * 4 * NT,
-                                          sm, seq, seq0);
+            stage_tile_tma<NT, KIND, PLM>(&I->mapB, &I->mapA, I->A, g, ph, c1, c2, c3, tm, tl.y, tl.z,
+                                          tl.w, (unsigned)I->tiles, dyn, dyn + kRing * 4 * NT, sm,
+                                          seq, seq0);
     }
 }
 
@@ -2441,7 +2440,7 @@ void launch_stage2d(const Ctx& c, const double* uc, const double* u0, double* ou
 }
 
 template <int NT, int KIND, bool PLM>
-static void launch_ens_stage_k(const gk::EnsInst* inst, const int2* tiles, int ntiles,
+static void launch_ens_stage_k(const gk::EnsInst* inst, const int4* tiles, int ntiles,
                                unsigned* counter, double c1, double c2, double c3, int ctas,
                                cudaStream_t s) {
     const size_t dyn = stage_dyn_bytes<NT, (KIND >= 1)>();
@@ -2453,7 +2452,7 @@ static void launch_ens_stage_k(const gk::EnsInst* inst, const int2* tiles, int n
 }
 
 template <int NT>
-static void launch_ens_stage_nt(int kind, int plm, const gk::EnsInst* inst, const int2* tiles,
+static void launch_ens_stage_nt(int kind, int plm, const gk::EnsInst* inst, const int4* tiles,
                                 int ntiles, unsigned* counter, double c1, double c2, double c3,
                                 cudaStream_t s) {
     const int ctas = std::min(ntiles, 148 * gk::stage_ctas(NT, !GK_FASTMATH));
@@ -2466,7 +2465,7 @@ static void launch_ens_stage_nt(int kind, int plm, const gk::EnsInst* inst, cons
     }
 }
 
-void launch_ens_stage(int threads, int kind, int plm, const gk::EnsInst* inst, const int2* tiles,
+void launch_ens_stage(int threads, int kind, int plm, const gk::EnsInst* inst, const int4* tiles,
                       int ntiles, unsigned* counter, double c1, double c2, double c3,
                       cudaStream_t s) {
     if (threads == 64) launch_ens_stage_nt<64>(kind, plm, inst, tiles, ntiles, counter, c1, c2, c3, s);

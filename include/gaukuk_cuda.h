@@ -259,8 +259,9 @@ int gk_set_tiling(gk_handle* h, int threads, int rows);
 typedef struct gk_ensemble gk_ensemble;
 int gk_ens_create(gk_handle* const* handles, int n, gk_ensemble** out);
 void gk_ens_destroy(gk_ensemble* e);
-/* threads per CTA (64, 128, 256) for all instances; rows: one entry per
- * instance, or NULL to keep the current ones (default 16). */
+/* threads per CTA (64, 128, 256) for all instances; rows of a tile: one entry
+ * per instance, or NULL to keep the current ones (default 16).  The tiles of
+ * the last, partly filled wave are cut shorter. */
 int gk_ens_set_tiling(gk_ensemble* e, int threads, const int* rows);
 /* Sim::Advance(dtoutput) on every instance, each from its own time. */
 int gk_ens_advance(gk_ensemble* e, double dtoutput);
