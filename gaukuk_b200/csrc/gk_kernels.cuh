@@ -107,8 +107,9 @@ __device__ __forceinline__ long long fidx(const Geom& g, int k, int j, int i) {
 // direction each ghost depends on one active cell, so all sides fill in one
 // launch.  blockIdx.y = 2*dir + side.
 // Outflow side (outflow.cpp:36-60): clamp inflow momentum, floor e_int at 1e-16.
+// The momentum is picked by compares: an index would put q into local memory.
 __device__ __forceinline__ void outflow_ghost(double (&q)[5], int mom, int side, const Phys& ph) {
-    double mt = q[mom];
+    double mt = mom == gk::S_MTX ? q[gk::S_MTX] : (mom == gk::S_MTY ? q[gk::S_MTY] : q[gk::S_MTZ]);
     double mc = side == 0 ? smin(mt, 0.0) : smax(mt, 0.0);
     double rho = smax(q[gk::S_DEN], ph.dmin);
     double rhoInv = 1.0 / rho;
@@ -117,18 +118,21 @@ __device__ __forceinline__ void outflow_ghost(double (&q)[5], int mom, int side,
     double eint = q[gk::S_ENG] - keOld;
     eint = smax(eint, 1e-16);
     q[gk::S_DEN] = rho;
-    q[mom] = mc;
+    if (mom == gk::S_MTX) q[gk::S_MTX] = mc;
+    else if (mom == gk::S_MTY) q[gk::S_MTY] = mc;
+    else q[gk::S_MTZ] = mc;
     q[gk::S_ENG] = eint + keNew;
 }
 // One ghost cell (id enumerates ghost layer fastest, then the transverse
 // active cells) of side `side` in direction `dir`, every variable.
 __device__ __forceinline__ void bc_fill_one(double* __restrict__ u, const Geom& g, const Phys& ph,
-                                            int dir, int side, long long id) {
+                                            int dir, int side, unsigned id) {
     const int n3[3] = {g.nx, g.ny, g.nz};
     const int type = ph.bc[2 * dir + side];
-    const int ta = dir == 0 ? g.ny : g.nx;
-    const int gi = (int)(id % g.ng);
-    const long long r = id / g.ng;
+    // 32-bit indices: a side has fewer than 2^32 ghosts
+    const unsigned ta = dir == 0 ? g.ny : g.nx;
+    const int gi = (int)(id % (unsigned)g.ng);
+    const unsigned r = id / (unsigned)g.ng;
     const int a = (int)(r % ta), b = (int)(r / ta);
     const int e = g.ng + n3[dir];
     const int gc = side == 0 ? gi : e + gi;  // ghost coordinate along dir
@@ -155,7 +159,9 @@ __device__ __forceinline__ void bc_fill_one(double* __restrict__ u, const Geom& 
     for (int v = 0; v < 5; ++v) q[v] = u[v * g.vstride + src];
     const int mom = dir == 0 ? gk::S_MTX : (dir == 1 ? gk::S_MTY : gk::S_MTZ);
     if (type == 2) {
-        q[mom] = -q[mom];
+        if (mom == gk::S_MTX) q[gk::S_MTX] = -q[gk::S_MTX];
+        else if (mom == gk::S_MTY) q[gk::S_MTY] = -q[gk::S_MTY];
+        else q[gk::S_MTZ] = -q[gk::S_MTZ];
     } else if (type == 3) {
         outflow_ghost(q, mom, side, ph);
     }
@@ -2165,9 +2171,10 @@ static inline int stage3d_nt(const Geom& g) {
 void launch_zflux(const Ctx& c, const double* u, double* F3, cudaStream_t s) {
     const Geom& g = c.g;
     const unsigned bx = (g.nx + kZX - 1) / kZX, by = (g.ny + kZY - 1) / kZY;
-    // faces per thread; nz + 1 faces in all
-    const int zseg = march_length(g.nz + 1, 48, (long long)bx * by, 148LL * 4, 1.5);
-    dim3 grid(bx, by, (g.nz + 1 + zseg - 1) / zseg);
+    // faces per thread, of nz + 1 (or the nz differences)
+    const int n = kZDiff ? g.nz : g.nz + 1;
+    const int zseg = march_length(n, 48, (long long)bx * by, 148LL * 4, kZDiff ? 2.5 : 1.5);
+    dim3 grid(bx, by, (n + zseg - 1) / zseg);
     if (c.ph.plm) k_zflux<true><<<grid, 128, 0, s>>>(u, F3, g, c.ph, c.tm, zseg);
     else k_zflux<false><<<grid, 128, 0, s>>>(u, F3, g, c.ph, c.tm, zseg);
 }
