@@ -213,6 +213,17 @@ __global__ void __launch_bounds__(128)
     }
 }
 
+// An 8-byte copy from global to the thread's own shared word, in flight until
+// copies_wait (no registers, no barrier).  The x-y stage's row inputs held 15-20
+// doubles in registers in fast mode (256^3: 2.01 -> 1.99 ms per step without) and
+// were loaded at their use in parity mode.
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ------------------------------------------------------------ x-y plane stage
 // THREE = false: out = c1*uc - c2*dF (stage 1); true: out = c1*u0 + c2*uc -
 // c3*dF.  out never aliases uc (neighbours of uc are read while out is
@@ -241,6 +252,9 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
     __shared__ double sP[5][NT];
     __shared__ double sXL[5][NT];
     __shared__ double sF[5][NT];
+    // rows of sIn: z-flux difference or lower z flux, raw state, base state, upper z flux
+    constexpr int kB0 = ZF ? 5 : 0, kIn = kB0 + (THREE ? 10 : 5) + (ZF && !kZDiff ? 5 : 0);
+    __shared__ double sIn[kIn][NT];
     const double dt = tm->dt;
     const double dtdx = dt * g.dxRec, dtdy = dt * g.dyRec, dtdz = dt * g.dzRec;
     const int t = threadIdx.x;
@@ -284,27 +298,20 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
     for (int f = y0 + 1; f <= y1; ++f) {
         const Q5 Q1 = Qn;
         if (f + 2 <= y1 + 1) Qn = load5(uc, g, at(f + 2));
-        // fast mode: the z-flux differences of cell row f-1, and its base
-        // state, are loaded here so that they arrive while the row's Riemann
-        // problems are solved (parity mode's longer IEEE sequences leave no
-        // registers for them: it loads them where they are used)
-        double dz[5], zlo[5], b0[5];  // dz: the z-flux difference, or the upper flux (zlo: the lower)
-        constexpr bool kEarly = GK_FASTMATH;
-        auto load_row_inputs = [&]() {
+        // what the update of cell row f-1 takes beside the fluxes: its z fluxes
+        // (or their difference), base state and raw state, copied to this
+        // thread's own shared words while the row's Riemann problems are solved
+        if (do_cell) {
             const long long fc = ZF ? fidx(g, k, f - 1, xi) : 0;
             const long long c = at(f - 1);
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
-                if (ZF && kZDiff) {
-                    dz[v] = __ldg(F3 + v * g.fvstride + fc);
-                } else if (ZF) {
-                    zlo[v] = __ldg(F3 + v * g.fvstride + fc);
-                    dz[v] = __ldg(F3 + v * g.fvstride + fc + g.fkstride);
-                }
-                b0[v] = THREE ? u0[v * g.vstride + c] : uc[v * g.vstride + c];
+                if (ZF) copy8(&sIn[v][t], F3 + v * g.fvstride + fc);
+                if (ZF && !kZDiff) copy8(&sIn[kIn - 5 + v][t], F3 + v * g.fvstride + fc + g.fkstride);
+                copy8(&sIn[kB0 + v][t], uc + v * g.vstride + c);
+                if (THREE) copy8(&sIn[kB0 + 5 + v][t], u0 + v * g.vstride + c);
             }
-        };
-        if (kEarly && do_cell) load_row_inputs();
+        }
         bool bad;  // parity mode: a quotient of this phase is out of range
         SlopeRange rg;
         clear(rg);
@@ -356,16 +363,17 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
         __syncthreads();
         if (do_cell) {
             // update_cons.cpp (3D): (Fx(i+1)-Fx(i))*dtdx + (Fy(j+1)-Fy(j))*dtdy + (Fz(k+1)-Fz(k))*dtdz
-            if (!kEarly) load_row_inputs();
+            copies_wait();
             const long long c = at(f - 1);
             double r[5];
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
                 double dF = (sF[v][tr] - fx[v]) * dtdx;
-                if (ZF) dF = dF + (fy[v] - fyPrev[v]) * dtdy + (kZDiff ? dz[v] : dz[v] - zlo[v]) * dtdz;
+                if (ZF) dF = dF + (fy[v] - fyPrev[v]) * dtdy +
+                             (kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]) * dtdz;
                 else dF = dF + (fy[v] - fyPrev[v]) * dtdy;
-                if (THREE) r[v] = c1 * b0[v] + c2 * uc[v * g.vstride + c] - c3 * dF;
-                else r[v] = c1 * b0[v] - c2 * dF;
+                if (THREE) r[v] = c1 * sIn[kB0 + 5 + v][t] + c2 * sIn[kB0 + v][t] - c3 * dF;
+                else r[v] = c1 * sIn[kB0 + v][t] - c2 * dF;
             }
             floors5(r, ph, tm);
             if (LAST) {
