@@ -242,8 +242,10 @@ int build_ctx(gk_handle* h) {
     ph.gmRec = 1.0 / pd.gamma;
     ph.cq = 0.5 * (1 + ph.gmRec);
     ph.gm1Rec1 = ph.gm1Rec + 1.0;
-    ph.gcq = ph.gamma * ph.cq;
+    ph.hgcq = 0.5 * ph.gamma * ph.cq;
     ph.hgm1 = 0.5 * ph.gm1;
+    ph.hgm1_over = ph.hgm1 * (1.0 + 1e-12);
+    ph.pmin_over = ph.pmin * (1.0 + 1e-12);
     ph.ranged = pd.gamma < 1024.0 && ph.gm1Rec < 1048576.0;
     ph.cfl = pd.cfl;
     ph.dmin = pd.dfloor;

@@ -72,8 +72,10 @@ struct Shell {
 struct Phys {
     double gamma, gm1, gm1Rec, gmRec, cq;  // cq = 0.5*(1+1/gamma) (hllc.cpp:55-58)
     double gm1Rec1;                        // gm1Rec + 1: fast mode's E + p = p*gm1Rec1 + rho k/2
-    double gcq;                            // gamma*cq: fast mode's gamma X = gamma p + gcq max(p* - p, 0)
+    double hgcq;                           // gamma*cq/2: fast mode's gamma X = gamma p + hgcq max(2p* - 2p, 0)
     double hgm1;                           // (gamma-1)/2: fast mode's conversion
+    double hgm1_over, pmin_over;           // hgm1 and pmin, 1e-12 larger: fast mode's pressure
+                                           // floor without a reciprocal (floors4_inv)
     int ranged;                            // gamma in the range parity mode's branch-free
                                            // division is built for (gk_physics.cuh)
     double cfl, dmin, pmin;

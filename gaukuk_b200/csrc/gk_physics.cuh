@@ -306,22 +306,25 @@ __device__ __forceinline__ void hllc_any(double denl, double vxl, double vyl, do
     double al = sqrt(GK_DIV(gamma * prel, denl));
     double ar = sqrt(GK_DIV(gamma * prer, denr));
 #endif
-    double prePVRS = 0.5 * (prel + prer) - 0.125 * (vxr - vxl) * (denl + denr) * (al + ar);
-    prePVRS = GK_MAX0(prePVRS);
 #if GK_FASTMATH
+    // 2p* of the PVRS estimate; max(p*, 0) is not taken, as only max(p* - p, 0)
+    // of positive pressures p is used
+    const double pvrs2 = fma(-0.25 * ((vxr - vxl) * (denl + denr)), al + ar, prel + prer);
     // a*q = sqrt(gamma p/rho) * sqrt(1 + cq max(p*/p - 1, 0)) = sqrt(gamma X/rho)
     // with X = p + cq max(p* - p, 0): one root per side, no quotient.
     // Branch-free on purpose: a skip when p* <= p (as in parity mode) was
     // measured slower, because it splits the straight-line code in which the
     // x- and y-face solves of a row interleave.
-    const double gxl = fma(ph.gcq, GK_MAX0(prePVRS - prel), gpl);
-    const double gxr = fma(ph.gcq, GK_MAX0(prePVRS - prer), gpr);
+    const double gxl = fma(ph.hgcq, GK_MAX0(fma(-2.0, prel, pvrs2)), gpl);
+    const double gxr = fma(ph.hgcq, GK_MAX0(fma(-2.0, prer, pvrs2)), gpr);
     // S - v = -+ gX rsqrt(gX rho), so rho (S - v) = -+ (gX rho) rsqrt(gX rho)
     const double xl = gxl * denl, xr = gxr * denr;
     const double rl = rsqrt_nr(xl), rr = rsqrt_nr(xr);
     double sl = vxl - gxl * rl;
     double sr = vxr + gxr * rr;
 #else
+    double prePVRS = 0.5 * (prel + prer) - 0.125 * (vxr - vxl) * (denl + denr) * (al + ar);
+    prePVRS = GK_MAX0(prePVRS);
     double ql, qr;
     // q = sqrt(1 + 0.5*(1+1/gamma)*max(p*/p - 1, 0)) is exactly 1 whenever
     // p* <= p with p > 0, so the division and root are skipped there.

@@ -257,6 +257,10 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
     __shared__ double sIn[kIn][NT];
     const double dt = tm->dt;
     const double dtdx = dt * g.dxRec, dtdy = dt * g.dyRec, dtdz = dt * g.dzRec;
+#if GK_FASTMATH
+    const double cx = THREE ? c3 * dtdx : dtdx, cy = THREE ? c3 * dtdy : dtdy;
+    const double cz = THREE ? c3 * dtdz : dtdz;
+#endif
     const int t = threadIdx.x;
     const int tl = t > 0 ? t - 1 : 0;
     const int tr = t < NT - 1 ? t + 1 : t;
@@ -368,18 +372,27 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
             double r[5];
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
+                const double u0v = THREE ? sIn[kB0 + 5 + v][t] : 0.0, q = sIn[kB0 + v][t];
+#if GK_FASTMATH
+                // each flux difference into the sum in one fused multiply-add
+                r[v] = stage_value<THREE>(c1, c2, cx, cy, u0v, q, sF[v][tr] - fx[v], fy[v] - fyPrev[v]);
+                if (ZF) r[v] = fma(-(kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]), cz, r[v]);
+#else
                 double dF = (sF[v][tr] - fx[v]) * dtdx;
                 if (ZF) dF = dF + (fy[v] - fyPrev[v]) * dtdy +
                              (kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]) * dtdz;
                 else dF = dF + (fy[v] - fyPrev[v]) * dtdy;
-                if (THREE) r[v] = c1 * sIn[kB0 + 5 + v][t] + c2 * sIn[kB0 + v][t] - c3 * dF;
-                else r[v] = c1 * sIn[kB0 + v][t] - c2 * dF;
+                if (THREE) r[v] = c1 * u0v + c2 * q - c3 * dF;
+                else r[v] = c1 * q - c2 * dF;
+#endif
             }
-            floors5(r, ph, tm);
+            constexpr bool SPEED = ZF && LAST == 1;
+            const double speed = floors5_speed<SPEED>(r, ph, tm);
             if (LAST) {
                 if (LAST == 2) kick_cell<false>(r, g, ph, dt, tm->t, 1, xi, f - 1, k);
-                const double local = cell_cmax(r[gk::S_DEN], r[gk::S_MTX], r[gk::S_MTY],
-                                               r[gk::S_MTZ], r[gk::S_ENG], ph, ZF || has_z);
+                const double local = SPEED ? speed
+                                           : cell_cmax(r[gk::S_DEN], r[gk::S_MTX], r[gk::S_MTY],
+                                                       r[gk::S_MTZ], r[gk::S_ENG], ph, ZF || has_z);
                 const unsigned long long b = (unsigned long long)__double_as_longlong(local);
                 cbest = b > cbest ? b : cbest;
             }
