@@ -2330,26 +2330,29 @@ void launch_stage3d(const Ctx& c, const double* uc, const double* u0, double* ou
     }
 }
 
+template <int KIND, bool PLM>
+static void launch_row_kind(const Ctx& c, double* uc, const double* u0, double* out, double c1, double c2,
+                            double c3, cudaStream_t s) {
+    const int tiles = (c.g.nx + kRowThreads - 5) / (kRowThreads - 4);
+    if (tiles > 148 * kRowCtas)
+        k_row_stage<KIND, PLM, kRowCtasLong><<<min(tiles, 148 * kRowCtasLong), kRowThreads, 0, s>>>(
+            uc, u0, out, c.g, c.ph, c1, c2, c3, c.tm, c.has_vz, tiles);
+    else
+        k_row_stage<KIND, PLM, kRowCtas><<<tiles, kRowThreads, 0, s>>>(uc, u0, out, c.g, c.ph, c1, c2, c3,
+                                                                      c.tm, c.has_vz, tiles);
+}
+
 // last: as launch_stage3d
 void launch_row_stage(const Ctx& c, double* uc, const double* u0, double* out, int last, double c1,
                       double c2, double c3, cudaStream_t s) {
-    const Geom& g = c.g;
-    const int tiles = (g.nx + kRowThreads - 5) / (kRowThreads - 4);
-    const int grid = min(tiles, 148 * (kStage3dThreadsPerSM / kRowThreads));
-#define GK_ROW(K, PL) \
-    k_row_stage<K, PL><<<grid, kRowThreads, 0, s>>>(uc, u0, out, g, c.ph, c1, c2, c3, c.tm, c.has_vz, tiles)
     const int kind = last ? 1 + last : (u0 ? 1 : 0);
-    if (c.ph.plm) {
-        if (kind == 0) GK_ROW(0, true);
-        else if (kind == 1) GK_ROW(1, true);
-        else if (kind == 2) GK_ROW(2, true);
-        else GK_ROW(3, true);
-    } else {
-        if (kind == 0) GK_ROW(0, false);
-        else if (kind == 1) GK_ROW(1, false);
-        else if (kind == 2) GK_ROW(2, false);
-        else GK_ROW(3, false);
-    }
+#define GK_ROW(K)                                                         \
+    if (c.ph.plm) launch_row_kind<K, true>(c, uc, u0, out, c1, c2, c3, s); \
+    else launch_row_kind<K, false>(c, uc, u0, out, c1, c2, c3, s)
+    if (kind == 0) { GK_ROW(0); }
+    else if (kind == 1) { GK_ROW(1); }
+    else if (kind == 2) { GK_ROW(2); }
+    else { GK_ROW(3); }
 #undef GK_ROW
 }
 

@@ -420,9 +420,14 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
 // (k_c2p, k_flux, k_update, k_kick, k_cfl), so the bits are the same; those
 // took 11 launches per RK2 step and converted every ghost row of the array
 // (262143 cells, parity: 90 us per step; FP64 alone needs 9).
-constexpr int kRowThreads = 128;
-template <int KIND, bool PLM>
-__global__ void __launch_bounds__(kRowThreads, kStage3dThreadsPerSM / kRowThreads)
+// CTAS: resident CTAs per SM.  A row with tiles for more than three per SM hides
+// its latency better with more, at fewer registers and without spills (5 in fast
+// mode, 4 in parity mode, which needs 128): 262143 cells, us per step, fast 18.5 ->
+// 17.2, parity 25.7 -> 24.4; 2^20 cells fast 53.1 -> 50.2.  Shorter rows keep three
+// (1100 cells, parity: 10.2, at four 10.35).
+constexpr int kRowThreads = 128, kRowCtas = 3, kRowCtasLong = GK_FASTMATH ? 5 : 4;
+template <int KIND, bool PLM, int CTAS>
+__global__ void __launch_bounds__(kRowThreads, CTAS)
     k_row_stage(double* uc, const double* u0, double* out, Geom g, Phys ph, double c1, double c2,
                 double c3, DevTime* tm, int has_z, int tiles) {
     if (!tm->active) return;
