@@ -501,16 +501,13 @@ __device__ __forceinline__ double floors4_inv(double (&r)[4], const Phys& ph, De
 }
 
 // Fast mode's new value of a variable from the base state u0, the stage's state
-// q (a first stage: c1 = c2 = 1, no u0) and the differences dx, dy of its
-// fluxes, each taken into the sum in one fused multiply-add (cx, cy: the last
-// coefficient times dtdx, dtdy).  With the floors' reciprocal left out, the CFL
-// speed sharing the floors' pressure and 2p* in the Riemann problem, a cell takes
-// 13-16 FP64 operations less than about 290 (KH 4096^2 938 -> 920 us per step,
-// RT 1024x3072 334 -> 327, 3D 256^3 2141 -> 2100).
+// q (a first stage has no u0) and the flux difference dF, which holds the last
+// coefficient already (cx, cy, cz in the callers).  c1 + c2 = 1 in every stage, so
+// c1 u0 + c2 q is q + c1 (u0 - q): two roundings at the size of the state, and none
+// of the bias of c1 + c2 = 1 - 2^-54 (thirds).
 template <bool THREE>
-__device__ __forceinline__ double stage_value(double c1, double c2, double cx, double cy, double u0,
-                                              double q, double dx, double dy) {
-    return fma(-dx, cx, fma(-dy, cy, THREE ? fma(c1, u0, c2 * q) : q));
+__device__ __forceinline__ double stage_value(double c1, double u0, double q, double dF) {
+    return THREE ? fma(c1, u0 - q, q - dF) : q - dF;
 }
 
 // Sim::UpdateCons (update_cons.cpp:11-68) of one RK stage: the flux
@@ -1522,10 +1519,10 @@ __global__ void __launch_bounds__(32 * (TY + 2), tile_ctas(TY))
             const W4 fr = get(&sm.xl[0][w], TY + 2, lr), fu = get(&sm.fy[0][w + 1], TY + 2, lane);
 #if GK_FASTMATH
             double r[4];
-            r[0] = stage_value<THREE>(c1, c2, cx, cy, b0.d, q.d, fr.r - fx.d, fu.r - fy.d);
-            r[1] = stage_value<THREE>(c1, c2, cx, cy, b0.mx, q.mx, fr.vx - fx.n, fu.vy - fy.t1);
-            r[2] = stage_value<THREE>(c1, c2, cx, cy, b0.my, q.my, fr.vy - fx.t1, fu.vx - fy.n);
-            r[3] = stage_value<THREE>(c1, c2, cx, cy, b0.e, q.e, fr.p - fx.e, fu.p - fy.e);
+            r[0] = stage_value<THREE>(c1, b0.d, q.d, (fr.r - fx.d) * cx + (fu.r - fy.d) * cy);
+            r[1] = stage_value<THREE>(c1, b0.mx, q.mx, (fr.vx - fx.n) * cx + (fu.vy - fy.t1) * cy);
+            r[2] = stage_value<THREE>(c1, b0.my, q.my, (fr.vy - fx.t1) * cx + (fu.vx - fy.n) * cy);
+            r[3] = stage_value<THREE>(c1, b0.e, q.e, (fr.p - fx.e) * cx + (fu.p - fy.e) * cy);
 #else
             const double dF0 = (fr.r - fx.d) * dtdx + (fu.r - fy.d) * dtdy;
             const double dF1 = (fr.vx - fx.n) * dtdx + (fu.vy - fy.t1) * dtdy;
@@ -1978,10 +1975,10 @@ __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CU
             double r[4];
             Q4 U0{};
             if (THREE) U0 = rowq0(f - 1);
-            r[0] = stage_value<THREE>(c1, c2, cx, cy, U0.d, Qm1.d, fr0.x - fx.d, fy.d - fyPrev.d);
-            r[1] = stage_value<THREE>(c1, c2, cx, cy, U0.mx, Qm1.mx, fr0.y - fx.n, fy.t1 - fyPrev.t1);
-            r[2] = stage_value<THREE>(c1, c2, cx, cy, U0.my, Qm1.my, fr1.x - fx.t1, fy.n - fyPrev.n);
-            r[3] = stage_value<THREE>(c1, c2, cx, cy, U0.e, Qm1.e, fr1.y - fx.e, fy.e - fyPrev.e);
+            r[0] = stage_value<THREE>(c1, U0.d, Qm1.d, (fr0.x - fx.d) * cx + (fy.d - fyPrev.d) * cy);
+            r[1] = stage_value<THREE>(c1, U0.mx, Qm1.mx, (fr0.y - fx.n) * cx + (fy.t1 - fyPrev.t1) * cy);
+            r[2] = stage_value<THREE>(c1, U0.my, Qm1.my, (fr1.x - fx.t1) * cx + (fy.n - fyPrev.n) * cy);
+            r[3] = stage_value<THREE>(c1, U0.e, Qm1.e, (fr1.y - fx.e) * cx + (fy.e - fyPrev.e) * cy);
 #else
             double dF0 = (fr0.x - fx.d) * dtdx + (fy.d - fyPrev.d) * dtdy;
             double dF1 = (fr0.y - fx.n) * dtdx + (fy.t1 - fyPrev.t1) * dtdy;

@@ -234,8 +234,8 @@ __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;
 // Resident threads per SM: 384, at up to 168 registers each (parity mode with
 // 40-72 bytes of spills).  Parity mode at 192^3: 1.74 ms per step, 1.72 at 256
 // threads without spills, which loses 10-30 % on small grids (64^3: 158 us
-// against 207); fast mode at 512 threads ran 2.28 -> 2.42 ms at 256^3 (its
-// early loads need the registers).
+// against 207); fast mode at 512 threads (128 registers, no spills) is no faster
+// at 256^3 (2.175 -> 2.162 ms) and slower on small grids (31x190x55 82 -> 88 us).
 constexpr int kStage3dThreadsPerSM = 384;
 // ZF = false: a 2D run with all five variables (one plane, no z fluxes): the
 // update is k_update's 2D expression.  A 2D run off the four-variable path
@@ -372,18 +372,17 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
             double r[5];
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
-                const double u0v = THREE ? sIn[kB0 + 5 + v][t] : 0.0, q = sIn[kB0 + v][t];
 #if GK_FASTMATH
-                // each flux difference into the sum in one fused multiply-add
-                r[v] = stage_value<THREE>(c1, c2, cx, cy, u0v, q, sF[v][tr] - fx[v], fy[v] - fyPrev[v]);
-                if (ZF) r[v] = fma(-(kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]), cz, r[v]);
+                double dF = (sF[v][tr] - fx[v]) * cx + (fy[v] - fyPrev[v]) * cy;
+                if (ZF) dF += (kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]) * cz;
+                r[v] = stage_value<THREE>(c1, THREE ? sIn[kB0 + 5 + v][t] : 0.0, sIn[kB0 + v][t], dF);
 #else
                 double dF = (sF[v][tr] - fx[v]) * dtdx;
                 if (ZF) dF = dF + (fy[v] - fyPrev[v]) * dtdy +
                              (kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]) * dtdz;
                 else dF = dF + (fy[v] - fyPrev[v]) * dtdy;
-                if (THREE) r[v] = c1 * u0v + c2 * q - c3 * dF;
-                else r[v] = c1 * q - c2 * dF;
+                if (THREE) r[v] = c1 * sIn[kB0 + 5 + v][t] + c2 * sIn[kB0 + v][t] - c3 * dF;
+                else r[v] = c1 * sIn[kB0 + v][t] - c2 * dF;
 #endif
             }
             constexpr bool SPEED = ZF && LAST == 1;
