@@ -257,10 +257,6 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
     __shared__ double sIn[kIn][NT];
     const double dt = tm->dt;
     const double dtdx = dt * g.dxRec, dtdy = dt * g.dyRec, dtdz = dt * g.dzRec;
-#if GK_FASTMATH
-    const double cx = THREE ? c3 * dtdx : dtdx, cy = THREE ? c3 * dtdy : dtdy;
-    const double cz = THREE ? c3 * dtdz : dtdz;
-#endif
     const int t = threadIdx.x;
     const int tl = t > 0 ? t - 1 : 0;
     const int tr = t < NT - 1 ? t + 1 : t;
@@ -373,9 +369,9 @@ __global__ void __launch_bounds__(NT, kStage3dThreadsPerSM / NT)
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
 #if GK_FASTMATH
-                double dF = (sF[v][tr] - fx[v]) * cx + (fy[v] - fyPrev[v]) * cy;
-                if (ZF) dF += (kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]) * cz;
-                r[v] = stage_value<THREE>(c1, THREE ? sIn[kB0 + 5 + v][t] : 0.0, sIn[kB0 + v][t], dF);
+                double dF = (sF[v][tr] - fx[v]) * dtdx + (fy[v] - fyPrev[v]) * dtdy;
+                if (ZF) dF += (kZDiff ? sIn[v][t] : sIn[kIn - 5 + v][t] - sIn[v][t]) * dtdz;
+                r[v] = stage_value<THREE>(c1, c2, c3, THREE ? sIn[kB0 + 5 + v][t] : 0.0, sIn[kB0 + v][t], dF);
 #else
                 double dF = (sF[v][tr] - fx[v]) * dtdx;
                 if (ZF) dF = dF + (fy[v] - fyPrev[v]) * dtdy +
