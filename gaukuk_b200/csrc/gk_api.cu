@@ -244,12 +244,12 @@ int build_ctx(gk_handle* h) {
     ph.gm1Rec1 = ph.gm1Rec + 1.0;
     ph.hgcq = 0.5 * ph.gamma * ph.cq;
     ph.hgm1 = 0.5 * ph.gm1;
-    ph.hgm1_over = ph.hgm1 * (1.0 + 1e-12);
-    ph.pmin_over = ph.pmin * (1.0 + 1e-12);
     ph.ranged = pd.gamma < 1024.0 && ph.gm1Rec < 1048576.0;
     ph.cfl = pd.cfl;
     ph.dmin = pd.dfloor;
     ph.pmin = pd.pfloor;
+    ph.hgm1_over = ph.hgm1 * (1.0 + 1e-12);
+    ph.pmin_over = ph.pmin * (1.0 + 1e-12);
     for (int d = 0; d < 3; ++d) ph.grav[d] = pd.grav[d];
     ph.has_grav = (pd.grav[0] != 0 || pd.grav[1] != 0 || pd.grav[2] != 0);
     ph.integrator = pd.integrator == 1 ? 1 : (pd.integrator == 3 ? 3 : 2);
