@@ -132,7 +132,12 @@ struct gk_handle {
     cudaEvent_t copied[5] = {};  // a variable's plane is in the caller's array
     int path = 0;  // 0 generic, 1 fused 2D
     bool uploaded = false;
-    int upload_step = 0;  // clock step at the last upload
+    // Whose ghost fill a frame carries: `strips` until the clock passes step
+    // strips_step, `strips_next` after it (see note_steps); strips_next is null
+    // while no steps have been enqueued since the upload.
+    const double* strips = nullptr;
+    const double* strips_next = nullptr;
+    int strips_step = 0;
     bool tiling_set = false;  // gk_set_tiling overrides the default tiling
     float* model = nullptr;   // learned flux correction (device), or null
     gk::FluxGate gate;
@@ -548,11 +553,11 @@ bool fused5(const gk_handle* h) {
     return h->path == 0 && h->ctx.g.ndim <= 2 && h->ctx.ph.integrator != 1 && !h->model;
 }
 
-// The buffer whose ghost fill a written frame carries (k_pack_state): the last
-// intermediate stage state's (B, or C where RK3's second stage lands in C).
-// Euler runs in place and keeps A's.
+// The buffer whose ghost fill a frame carries after a step on the handle's
+// present path (k_pack_state): the last intermediate stage state's (B, or C
+// where RK3's second stage lands in C).  Euler runs in place and keeps A's.
 const double* last_stage_buffer(const gk_handle* h) {
-    if (h->ctx.ph.integrator == 1) return nullptr;
+    if (h->ctx.ph.integrator == 1) return h->A;
     return h->ctx.ph.integrator == 3 && (h->path == 1 || h->path == 2 || fused5(h)) ? h->C : h->B;
 }
 
@@ -722,6 +727,22 @@ int pull_time(gk_handle* h) {
     return GK_OK;
 }
 
+// Called before steps are enqueued that leave their last ghost fill in `buf`.
+// Whether steps enqueued earlier, on another path, ran at all (the step limit
+// or the output time may have ended the run) decides whose strips are kept if
+// the new ones do not run: that is read from the clock, once per change.
+int note_steps(gk_handle* h, const double* buf) {
+    if (buf == h->strips_next) return GK_OK;
+    if (h->strips_next) {
+        const int rc = pull_time(h);
+        if (rc != GK_OK) return rc;
+        if (h->htm->step > h->strips_step) h->strips = h->strips_next;
+        h->strips_step = h->htm->step;
+    }
+    h->strips_next = buf;
+    return GK_OK;
+}
+
 // Transfers of a whole state.  The reference layout is dense (NVar x lenz x
 // leny x lenx), the device's rows are pitched and its slots ordered DEN, MTX,
 // MTY, ENG, MTZ.  Where the handle has the generic path's scratch W (1D, 3D,
@@ -747,7 +768,8 @@ __global__ void k_unpack_state(const double* __restrict__ src, double* __restric
 // with cons.Swap(consTemp) (rk2.cpp:21, rk3.cpp:27), so the written array
 // carries the ghost fill of the last intermediate stage state.  The ghost
 // strips of active rows, columns and planes therefore come from the stage
-// buffer `donor` once a step has been taken since the upload.
+// buffer of the last step that ran, or from the state itself where none has
+// since the upload (the handle's strips and strips_next).
 __device__ __forceinline__ bool from_donor(const gk::Geom& g, int fill_z, int k, int j, int i) {
     const bool ai = i >= g.ib && i < g.ie, aj = j >= g.jb && j < g.je, ak = k >= g.kb && k < g.ke;
     if (!ai && g.nx > 1) return aj && ak;
@@ -755,25 +777,25 @@ __device__ __forceinline__ bool from_donor(const gk::Geom& g, int fill_z, int k,
     if (!ak && g.nz > 1) return ai && aj && ((fill_z >> (k < g.kb ? 0 : 1)) & 1);
     return false;
 }
-__global__ void k_pack_state(const double* __restrict__ u, const double* __restrict__ donor,
+__global__ void k_pack_state(const double* u, const double* strips, const double* strips_next,
                              double* __restrict__ dst, gk::Geom g, int fill_z,
-                             const gk::DevTime* __restrict__ tm, int upload_step) {
+                             const gk::DevTime* __restrict__ tm, int strips_step) {
     constexpr int slot[5] = {gk::S_DEN, gk::S_MTX, gk::S_MTY, gk::S_MTZ, gk::S_ENG};
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.lenx) return;
-    const bool use = donor && tm->step > upload_step;
+    const double* donor = tm->step > strips_step ? strips_next : strips;
     const int rows = g.nzs * g.leny;
     for (int r = blockIdx.y; r < 5 * rows; r += gridDim.y) {
         const int n = r / rows, q = r - n * rows;
-        const bool other = use && from_donor(g, fill_z, g.kofs + q / g.leny, q % g.leny, i);
+        const bool other = from_donor(g, fill_z, g.kofs + q / g.leny, q % g.leny, i);
         dst[(long long)r * g.lenx + i] =
             (other ? donor : u)[slot[n] * g.vstride + (long long)q * g.pitch + i];
     }
 }
 // 2D: per slot the x strips [side][row][2], then the y strips [side][2][column].
-__global__ void k_gather_strips(const double* __restrict__ u, const double* __restrict__ donor,
+__global__ void k_gather_strips(const double* __restrict__ strips, const double* __restrict__ strips_next,
                                 double* __restrict__ dst, gk::Geom g,
-                                const gk::DevTime* __restrict__ tm, int upload_step) {
+                                const gk::DevTime* __restrict__ tm, int strips_step) {
     const int nx4 = 2 * g.ng * g.ny, total = nx4 + 2 * g.ng * g.nx;
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= total) return;
@@ -787,7 +809,7 @@ __global__ void k_gather_strips(const double* __restrict__ u, const double* __re
         j = (side ? g.je : 0) + r / g.nx;
         i = g.ib + r % g.nx;
     }
-    const double* src = donor && tm->step > upload_step ? donor : u;
+    const double* src = tm->step > strips_step ? strips_next : strips;
     dst[(long long)blockIdx.y * total + id] =
         src[blockIdx.y * g.vstride + (long long)j * g.pitch + i];
 }
@@ -1028,7 +1050,9 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
     rc = pull_time(h);
     if (rc != GK_OK) return rc;
     h->uploaded = true;
-    h->upload_step = h->htm->step;
+    h->strips = h->A;
+    h->strips_next = nullptr;
+    h->strips_step = h->htm->step;
     if (h->htm->status) return fail(h, GK_ERR_NONFINITE, "non-finite state in the uploaded array");
     return GK_OK;
 }
@@ -1044,19 +1068,18 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
     // download leaves the caller's plane as it is.
     const bool skip_mtz = !zero_other_planes && h->mtz_plane_zero && h->path == 1 &&
                           !h->ctx.ph.fixed_bd;
-    // whose ghost strips the frame carries; 1D y rows follow the reference's
-    // in-place order and keep A's (from_donor)
-    const double* donor = last_stage_buffer(h);
+    // 1D y rows follow the reference's in-place order and keep A's (from_donor)
+    const double* strips_next = h->strips_next ? h->strips_next : h->strips;
     const size_t len = (size_t)g.nzs * g.leny * g.lenx, total = g.ndim == 2 ? strip_doubles(g) : 0;
     const bool dense = h->path != 1;
     const int slots = skip_mtz ? 4 : 5;  // MTZ's is the last
     h->io_down = 0;
     if (dense) {
-        k_pack_state<<<rows_grid(g), 256, 0, h->stream>>>(h->A, donor, h->W, g, h->ctx.ph.fill_z, h->tm,
-                                                          h->upload_step);
+        k_pack_state<<<rows_grid(g), 256, 0, h->stream>>>(h->A, h->strips, strips_next, h->W, g,
+                                                          h->ctx.ph.fill_z, h->tm, h->strips_step);
     } else {
         k_gather_strips<<<dim3((unsigned)((total + 127) / 128), slots), 128, 0, h->stream>>>(
-            h->A, donor, h->dstrips, g, h->tm, h->upload_step);
+            h->strips, strips_next, h->dstrips, g, h->tm, h->strips_step);
     }
     GK_CUDA(h, cudaGetLastError());
     if (!dense) {
@@ -1134,6 +1157,8 @@ static void refill_ghosts(gk_handle* h) {
 // host), every step enqueued and finished in turn.
 static int run_loop_host(gk_handle* h, double dtoutput, int nsteps) {
     h->host_fill_rc = GK_OK;
+    int rc = note_steps(h, last_stage_buffer(h));
+    if (rc != GK_OK) return rc;
     h->ks->begin(h->ctx, dtoutput, nsteps, h->stream);
     GK_CUDA(h, cudaGetLastError());
     for (int i = 0; nsteps <= 0 || i < nsteps; ++i) {
@@ -1161,6 +1186,7 @@ static int run_loop(gk_handle* h, double dtoutput, int nsteps, bool wait) {
     const int rest = nsteps > 0 && 2 * (nsteps % per) <= per ? nsteps % per : 0;
     const int graphs = nsteps > 0 ? (nsteps - rest + per - 1) / per : 1;
     int rc = graphs > 0 ? ensure_graph(h) : GK_OK;
+    if (rc == GK_OK) rc = note_steps(h, last_stage_buffer(h));
     if (rc != GK_OK) return rc;
     h->ks->begin(h->ctx, dtoutput, nsteps, h->stream);
     refill_ghosts(h);
@@ -1324,6 +1350,7 @@ int gk_graph_info(gk_handle* h, int* steps_per_graph, int* launches_per_step) {
 int gk_profile_steps(gk_handle* h, int nsteps, char* names, int names_cap, double* total_ms,
                      int* launches, int cap, int* n) {
     int rc = check_ready(h);
+    if (rc == GK_OK) rc = note_steps(h, last_stage_buffer(h));
     if (rc != GK_OK) return rc;
     h->ks->begin(h->ctx, 0.0, nsteps, h->stream);
     refill_ghosts(h);
@@ -1606,6 +1633,8 @@ int ens_run(gk_ensemble* e, double dtoutput, int nsteps, bool wait) {
     for (gk_handle* h : e->h) GK_ECUDA(e, cudaStreamSynchronize(h->stream));
     int rc = ens_graph(e);
     if (rc != GK_OK) return rc;
+    for (gk_handle* h : e->h)
+        if ((rc = note_steps(h, h->B)) != GK_OK) return efail(e, rc, h->err);
     e->ks->ens_begin(e->dinst, e->n, dtoutput, nsteps, e->stream);
     GK_ECUDA(e, cudaGetLastError());
     if (nsteps > 0) {
@@ -1812,6 +1841,7 @@ extern "C" int gk_tap_substeps(gk_handle* h, int nsub, double dt_sub, int ratio,
     rc = alloc_generic(h);
     if (rc != GK_OK) return rc;
     h->ghosts_dirty = true;  // the taps advance A on the generic path
+    if ((rc = note_steps(h, h->B)) != GK_OK) return rc;
     const int nxc = g.nx / ratio, nyc = g.ny / ratio;
     const size_t nacc = (size_t)4 * nxc * nyc;
     double* acc = nullptr;
@@ -2335,6 +2365,8 @@ int slabs_check_ready(gk_slabs* G) {
 int slabs_run(gk_slabs* G, double dtoutput, int nsteps) {
     int rc = slabs_reduce(G, 1);
     if (rc != GK_OK) return rc;
+    for (gk_handle* h : G->s)
+        if ((rc = note_steps(h, last_stage_buffer(h))) != GK_OK) return sfail(G, rc, h->err);
     const KernelSet& k = *G->s[0]->ks;
     for (gk_handle* h : G->s) k.begin(h->ctx, dtoutput, nsteps, G->stream);
     gk_handle* h0 = G->s[0];
