@@ -132,12 +132,13 @@ struct gk_handle {
     cudaEvent_t copied[5] = {};  // a variable's plane is in the caller's array
     int path = 0;  // 0 generic, 1 fused 2D
     bool uploaded = false;
-    // Whose ghost fill a frame carries: `strips` until the clock passes step
-    // strips_step, `strips_next` after it (see note_steps); strips_next is null
+    // Whose ghost fill a frame carries: `strips` while no more than strips_taken
+    // steps have been taken since the upload (DevTime::nlog; the step number can
+    // be set), `strips_next` after that (see note_steps); strips_next is null
     // while no steps have been enqueued since the upload.
     const double* strips = nullptr;
     const double* strips_next = nullptr;
-    int strips_step = 0;
+    int strips_taken = 0;
     bool tiling_set = false;  // gk_set_tiling overrides the default tiling
     float* model = nullptr;   // learned flux correction (device), or null
     gk::FluxGate gate;
@@ -736,8 +737,8 @@ int note_steps(gk_handle* h, const double* buf) {
     if (h->strips_next) {
         const int rc = pull_time(h);
         if (rc != GK_OK) return rc;
-        if (h->htm->step > h->strips_step) h->strips = h->strips_next;
-        h->strips_step = h->htm->step;
+        if (h->htm->nlog > h->strips_taken) h->strips = h->strips_next;
+        h->strips_taken = h->htm->nlog;
     }
     h->strips_next = buf;
     return GK_OK;
@@ -779,11 +780,11 @@ __device__ __forceinline__ bool from_donor(const gk::Geom& g, int fill_z, int k,
 }
 __global__ void k_pack_state(const double* u, const double* strips, const double* strips_next,
                              double* __restrict__ dst, gk::Geom g, int fill_z,
-                             const gk::DevTime* __restrict__ tm, int strips_step) {
+                             const gk::DevTime* __restrict__ tm, int strips_taken) {
     constexpr int slot[5] = {gk::S_DEN, gk::S_MTX, gk::S_MTY, gk::S_MTZ, gk::S_ENG};
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.lenx) return;
-    const double* donor = tm->step > strips_step ? strips_next : strips;
+    const double* donor = tm->nlog > strips_taken ? strips_next : strips;
     const int rows = g.nzs * g.leny;
     for (int r = blockIdx.y; r < 5 * rows; r += gridDim.y) {
         const int n = r / rows, q = r - n * rows;
@@ -795,7 +796,7 @@ __global__ void k_pack_state(const double* u, const double* strips, const double
 // 2D: per slot the x strips [side][row][2], then the y strips [side][2][column].
 __global__ void k_gather_strips(const double* __restrict__ strips, const double* __restrict__ strips_next,
                                 double* __restrict__ dst, gk::Geom g,
-                                const gk::DevTime* __restrict__ tm, int strips_step) {
+                                const gk::DevTime* __restrict__ tm, int strips_taken) {
     const int nx4 = 2 * g.ng * g.ny, total = nx4 + 2 * g.ng * g.nx;
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= total) return;
@@ -809,7 +810,7 @@ __global__ void k_gather_strips(const double* __restrict__ strips, const double*
         j = (side ? g.je : 0) + r / g.nx;
         i = g.ib + r % g.nx;
     }
-    const double* src = tm->step > strips_step ? strips_next : strips;
+    const double* src = tm->nlog > strips_taken ? strips_next : strips;
     dst[(long long)blockIdx.y * total + id] =
         src[blockIdx.y * g.vstride + (long long)j * g.pitch + i];
 }
@@ -1052,7 +1053,7 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
     h->uploaded = true;
     h->strips = h->A;
     h->strips_next = nullptr;
-    h->strips_step = h->htm->step;
+    h->strips_taken = 0;
     if (h->htm->status) return fail(h, GK_ERR_NONFINITE, "non-finite state in the uploaded array");
     return GK_OK;
 }
@@ -1076,10 +1077,10 @@ static int download(gk_handle* h, double* cons, bool zero_other_planes) {
     h->io_down = 0;
     if (dense) {
         k_pack_state<<<rows_grid(g), 256, 0, h->stream>>>(h->A, h->strips, strips_next, h->W, g,
-                                                          h->ctx.ph.fill_z, h->tm, h->strips_step);
+                                                          h->ctx.ph.fill_z, h->tm, h->strips_taken);
     } else {
         k_gather_strips<<<dim3((unsigned)((total + 127) / 128), slots), 128, 0, h->stream>>>(
-            h->strips, strips_next, h->dstrips, g, h->tm, h->strips_step);
+            h->strips, strips_next, h->dstrips, g, h->tm, h->strips_taken);
     }
     GK_CUDA(h, cudaGetLastError());
     if (!dense) {
@@ -1841,7 +1842,7 @@ extern "C" int gk_tap_substeps(gk_handle* h, int nsub, double dt_sub, int ratio,
     rc = alloc_generic(h);
     if (rc != GK_OK) return rc;
     h->ghosts_dirty = true;  // the taps advance A on the generic path
-    if ((rc = note_steps(h, h->B)) != GK_OK) return rc;
+    h->strips = h->strips_next = h->B;  // the log does not count its steps
     const int nxc = g.nx / ratio, nyc = g.ny / ratio;
     const size_t nacc = (size_t)4 * nxc * nyc;
     double* acc = nullptr;
