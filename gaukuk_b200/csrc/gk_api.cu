@@ -442,7 +442,7 @@ int stage_tile_rows(const gk::Geom& g, int threads, int rows, bool parity) {
 // Path 2, the 3D stage (z fluxes, then one fused x-y stage per plane),
 // applies to 3D RK2/RK3 runs (forward Euler updates in place, which the
 // fused stage cannot).  Path 3, a 1D run in one CTA or cluster (k_run1d, many steps
-// per launch), applies to 1D runs of up to 1024 cells per row (lenx) with
+// per launch), applies to 1D runs of 2 cells up to 1024 per row (lenx) with
 // the device's own ghost fills (copy, periodic, reflecting, outflow) and no
 // source term, learned correction or host routine.  Path 0 is generic.
 int choose_path(const gk_handle* h) {
@@ -451,7 +451,7 @@ int choose_path(const gk_handle* h) {
     if (c.g.ndim == 1) {
         bool own_fills = true;
         for (int s = 0; s < 2; ++s) own_fills = own_fills && c.ph.bc[s] >= 0 && c.ph.bc[s] <= 3;
-        return (c.g.lenx <= 1024 && own_fills && !c.ph.has_grav && c.ph.npoint == 0 &&
+        return (c.g.nx > 1 && c.g.lenx <= 1024 && own_fills && !c.ph.has_grav && c.ph.npoint == 0 &&
                 c.ph.nshell == 0 && !c.ph.fix_inner && !h->model && h->host_fills.empty() &&
                 env_int("GK_RUN1D", 1) != 0) ? 3 : 0;
     }
@@ -549,9 +549,10 @@ int run_host_fills(gk_handle* h, double* u) {
 // Whether a run on the generic path takes a fused stage of five variables: in
 // 2D the x-y stage without z fluxes (k_stage3d), in 1D the row stage
 // (k_row_stage).  RK2 and RK3; forward Euler updates in place, and the learned
-// correction as a pass needs the face-flux arrays.
+// correction as a pass needs the face-flux arrays; a single cell's ghosts are
+// filled one after the other (launch_bc).
 bool fused5(const gk_handle* h) {
-    return h->path == 0 && h->ctx.g.ndim <= 2 && h->ctx.ph.integrator != 1 && !h->model;
+    return h->path == 0 && h->ctx.g.ndim <= 2 && h->ctx.g.nx > 1 && h->ctx.ph.integrator != 1 && !h->model;
 }
 
 // The buffer whose ghost fill a frame carries after a step on the handle's
@@ -560,6 +561,21 @@ bool fused5(const gk_handle* h) {
 const double* last_stage_buffer(const gk_handle* h) {
     if (h->ctx.ph.integrator == 1) return h->A;
     return h->ctx.ph.integrator == 3 && (h->path == 1 || h->path == 2 || fused5(h)) ? h->C : h->B;
+}
+
+// A grid of one cell: some ghosts copy ghosts, so what an array's ghosts held
+// before a fill counts.  The reference swaps its two arrays after every step
+// (cons.Swap(consTemp)) where this library keeps the state in A, so the x ghosts
+// of A and B change places before every step but the first.
+__global__ void k_swap_x_ghosts(double* __restrict__ a, double* __restrict__ b, gk::Geom g,
+                                const gk::DevTime* __restrict__ tm) {
+    if (!tm->active || tm->nlog == 0 || threadIdx.x >= 10 * g.ng) return;
+    const int v = threadIdx.x / (2 * g.ng), q = threadIdx.x % (2 * g.ng);
+    const long long c = v * g.vstride + (g.kb - g.kofs) * g.kstride + (long long)g.jb * g.pitch +
+                        (q < g.ng ? q : g.nx + q);
+    const double t = a[c];
+    a[c] = b[c];
+    b[c] = t;
 }
 
 // One time step.  Kernel order per RK stage follows Sim::RK2_/RK3_/
@@ -594,6 +610,7 @@ void enqueue_step(gk_handle* h, Profiler* prof) {
     double* Cb = h->C;
     const int integ = c.ph.integrator;
     const double frac13 = 1.0 / 3.0;
+    if (c.g.nx == 1) GK_L(gk::K_BC, (k_swap_x_ghosts<<<1, 32, 0, s>>>(A, B, c.g, c.tm)));
     if (c.ph.has_grav || c.ph.npoint) GK_L(gk::K_KICK, k.kick(c, A, 0, s));
     if (h->path == 3) {
         // the whole step in one launch (ghost fills, stages, CFL, epilogue)
@@ -773,7 +790,7 @@ __global__ void k_unpack_state(const double* __restrict__ src, double* __restric
 // since the upload (the handle's strips and strips_next).
 __device__ __forceinline__ bool from_donor(const gk::Geom& g, int fill_z, int k, int j, int i) {
     const bool ai = i >= g.ib && i < g.ie, aj = j >= g.jb && j < g.je, ak = k >= g.kb && k < g.ke;
-    if (!ai && g.nx > 1) return aj && ak;
+    if (!ai) return aj && ak;
     if (!aj && g.ny > 1) return ai && ak;
     if (!ak && g.nz > 1) return ai && aj && ((fill_z >> (k < g.kb ? 0 : 1)) & 1);
     return false;
@@ -1344,7 +1361,8 @@ int gk_graph_info(gk_handle* h, int* steps_per_graph, int* launches_per_step) {
     } else if (h->path == 3) {
         per = 1;  // in a graph, one launch runs all of its steps
     } else {
-        per = (c.ph.has_grav || c.ph.npoint ? 2 : 0) + stages * (3 + inner + c.g.ndim) + 1;
+        per = (c.ph.has_grav || c.ph.npoint ? 2 : 0) + stages * (3 + inner + c.g.ndim) + 1 +
+              (c.g.nx == 1 ? 1 : 0);
     }
     if (steps_per_graph) *steps_per_graph = steps_per_graph_of(c.g);
     if (launches_per_step) *launches_per_step = per;

@@ -105,7 +105,7 @@ __device__ __forceinline__ long long fidx(const Geom& g, int k, int j, int i) {
 // boundary/{outflow_copy,periodic,reflective,outflow}.cpp.  Ghosts of active
 // rows/columns only; corners untouched.  With n >= nghost in every filled
 // direction each ghost depends on one active cell, so all sides fill in one
-// launch.  blockIdx.y = 2*dir + side.
+// launch (a grid of one cell: k_bc_one_cell).  blockIdx.y = 2*dir + side.
 // Outflow side (outflow.cpp:36-60): clamp inflow momentum, floor e_int at 1e-16.
 // The momentum is picked by compares: an index would put q into local memory.
 __device__ __forceinline__ void outflow_ghost(double (&q)[5], int mom, int side, const Phys& ph) {
@@ -184,6 +184,14 @@ __global__ void k_bc(double* __restrict__ u, Geom g, Phys ph, const DevTime* __r
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= count) return;
     bc_fill_one(u, g, ph, dir, side, id);
+}
+
+// A grid of one cell: the x sides of UpdateBD in its order, as ghosts are copied
+// from ghosts there.
+__global__ void k_bc_one_cell(double* __restrict__ u, Geom g, Phys ph, const DevTime* __restrict__ tm) {
+    if (!tm->active) return;
+    for (int side = 0; side < 2; ++side)
+        for (int gi = 0; gi < g.ng; ++gi) bc_fill_one(u, g, ph, 0, side, gi);
 }
 
 // Cell centres in Domain's order of operations (sim.cpp:36-41).
@@ -2184,12 +2192,14 @@ static inline dim3 cell_grid(const Geom& g, int threads) {
 
 void launch_bc(const Ctx& c, double* u, cudaStream_t s) {
     const Geom& g = c.g;
+    if (g.nx == 1) {  // then the other directions have one cell too
+        k_bc_one_cell<<<1, 1, 0, s>>>(u, g, c.ph, c.tm);
+        return;
+    }
     // size the grid for the directions that are filled only
-    long long m = 0;
-    if (g.nx > 1) m = max(m, (long long)g.ng * g.ny * g.nz);
+    long long m = (long long)g.ng * g.ny * g.nz;
     if (g.ny > 1) m = max(m, (long long)g.ng * g.nx * g.nz);
     if (g.nz > 1 && c.ph.fill_z) m = max(m, (long long)g.ng * g.nx * g.ny);
-    if (m == 0) return;
     const int sides = (g.nz > 1 && c.ph.fill_z) ? 6 : 4;
     dim3 grid((unsigned)((m + 127) / 128), sides);
     k_bc<<<grid, 128, 0, s>>>(u, g, c.ph, c.tm);
