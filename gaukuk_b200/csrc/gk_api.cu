@@ -899,10 +899,15 @@ bool host_all_zero(const double* p, size_t n) {
     return true;
 }
 
+// Whether a 1D or 2D run makes a z momentum that is zero at upload non-zero: a
+// point mass off the mid-plane and z gravity do, an immersed body writes it
+// (signed zeros in 2D) into its shell cells.
+bool makes_vz(const gk::Phys& ph) { return ph.npoint || ph.nshell || ph.grav[2] != 0; }
+
 // A change of the physics that kernels take by value: the captured graph
 // is rebuilt at the next launch, and the path follows.
 int physics_changed(gk_handle* h) {
-    if (h->ctx.ph.npoint || h->ctx.ph.nshell) h->ctx.has_vz = 1;  // see gk_upload_cons
+    if (makes_vz(h->ctx.ph)) h->ctx.has_vz = 1;
     if (h->gexec) {
         cudaGraphExecDestroy(h->gexec);
         h->gexec = nullptr;
@@ -1042,9 +1047,7 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
         GK_CUDA(h, cudaStreamSynchronize(h->stream));
         h->ctx.has_vz = flag;
     }
-    // a point mass off the mid-plane makes MTZ non-zero during the run; an
-    // immersed body writes MTZ (signed zeros in 2D) into its shell cells
-    if (h->ctx.ph.npoint || h->ctx.ph.nshell) h->ctx.has_vz = 1;
+    if (makes_vz(h->ctx.ph)) h->ctx.has_vz = 1;
     set_path(h);
     h->ctx.use_tma = env_int("GK_STAGE_TMA", 1) != 0;
     if (!h->tiling_set) {
