@@ -10,6 +10,7 @@
 // The host launches the graph repeatedly and only looks at `active` between
 // batches, so surplus launches cost one no-op kernel each.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -904,15 +905,24 @@ bool host_all_zero(const double* p, size_t n) {
 // (signed zeros in 2D) into its shell cells.
 bool makes_vz(const gk::Phys& ph) { return ph.npoint || ph.nshell || ph.grav[2] != 0; }
 
+// The captured graph holds launches that no longer fit: rebuilt at the next one.
+void drop_graph(gk_handle* h) {
+    if (!h->gexec) return;
+    cudaGraphExecDestroy(h->gexec);
+    h->gexec = nullptr;
+    h->graph_steps = 0;
+}
+
+// What an upload decides of the launches beside the path: v_z and the tile shape.
+std::array<int, 6> upload_choices(const gk::Ctx& c) {
+    return {c.has_vz, c.use_tma, c.stage_threads, c.h2d_rows, c.learn_rows, c.tile_rows};
+}
+
 // A change of the physics that kernels take by value: the captured graph
 // is rebuilt at the next launch, and the path follows.
 int physics_changed(gk_handle* h) {
     if (makes_vz(h->ctx.ph)) h->ctx.has_vz = 1;
-    if (h->gexec) {
-        cudaGraphExecDestroy(h->gexec);
-        h->gexec = nullptr;
-        h->graph_steps = 0;
-    }
+    drop_graph(h);
     if (h->uploaded) {
         set_path(h);
         if (h->path != 1) return alloc_generic(h);
@@ -1036,6 +1046,7 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
     }
     // Path: the fused kernel evolves four variables; it applies when the run
     // is 2D and MTZ is zero on every active cell (it then stays zero).
+    const auto before = upload_choices(h->ctx);
     h->ctx.has_vz = 1;
     if (g.ndim <= 2 && h->mtz_plane_zero) {
         h->ctx.has_vz = 0;
@@ -1060,6 +1071,7 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
         h->ctx.h2d_rows = h->tiling_rows;
         h->ctx.learn_rows = 0;
     }
+    if (upload_choices(h->ctx) != before) drop_graph(h);
     if (h->path != 1) {
         int rc = alloc_generic(h);
         if (rc != GK_OK) return rc;
