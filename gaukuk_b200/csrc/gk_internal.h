@@ -16,14 +16,18 @@
 
 namespace gk {
 
-// True the first time it is called for the current device with this mask:
-// kernel attributes (dynamic shared memory above 48 KB) are per device, so a
-// process that drives several GPUs sets them on each.
-inline bool first_on_device(std::atomic<unsigned long long>& mask) {
+// Runs `set` unless it has run for the current device with this mask: kernel
+// attributes (dynamic shared memory above 48 KB) are per device, so a process that
+// drives several GPUs sets them on each.  The mask is marked after `set`, so that
+// no thread launches before the attribute stands; two that come at once both set it.
+template <class F>
+inline void once_per_device(std::atomic<unsigned long long>& mask, F&& set) {
     int dev = 0;
     cudaGetDevice(&dev);
     const unsigned long long bit = 1ull << (dev & 63);
-    return (mask.fetch_or(bit) & bit) == 0;
+    if (mask.load(std::memory_order_acquire) & bit) return;
+    set();
+    mask.fetch_or(bit, std::memory_order_release);
 }
 
 // Resident CTAs per SM the fused 2D stage is compiled for at nt threads per

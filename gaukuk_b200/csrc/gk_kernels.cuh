@@ -2370,8 +2370,9 @@ template <bool HAS_Z, int NT, bool CLUSTER>
 static void launch_run1d_t(const Ctx& c, double* A, double* B, int nsteps, unsigned ctas, cudaStream_t s) {
     constexpr int bytes = (int)sizeof(Run1dShared<NT>);
     static std::atomic<unsigned long long> attr_set{0};
-    if (gk::first_on_device(attr_set))
+    gk::once_per_device(attr_set, [&] {
         cudaFuncSetAttribute(k_run1d<HAS_Z, NT, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    });
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2415,9 +2416,10 @@ static void launch_stage2d_tma(const Ctx& c, const CUtensorMap& mc, const CUtens
     dim3 grid((g.nx + NT - 5) / (NT - 4), (g.ny + rows - 1) / rows);
     const size_t dyn = stage_dyn_bytes<NT, (KIND >= 1)>();
     static std::atomic<unsigned long long> attr_set{0};
-    if (gk::first_on_device(attr_set))
+    gk::once_per_device(attr_set, [&] {
         cudaFuncSetAttribute(k_stage2d_tma<NT, KIND, PLM>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    });
     k_stage2d_tma<NT, KIND, PLM><<<grid, NT, dyn, s>>>(mc, m0, out, g, c.ph, c1, c2, c3, c.tm, rows);
 }
 
@@ -2445,9 +2447,10 @@ static void launch_stage2d_learn_k(const Ctx& c, const CUtensorMap& mc, const CU
     dim3 grid((g.nx + NT - 5) / (NT - 4), (g.ny + rows - 1) / rows);
     const size_t dyn = learn_dyn_bytes<NT, (KIND >= 1)>();
     static std::atomic<unsigned long long> attr_set{0};
-    if (gk::first_on_device(attr_set))
+    gk::once_per_device(attr_set, [&] {
         cudaFuncSetAttribute(k_stage2d_learn<NT, KIND, PLM>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    });
     k_stage2d_learn<NT, KIND, PLM><<<grid, NT, dyn, s>>>(mc, m0, out, g, c.ph, c1, c2, c3, c.tm, rows,
                                                          model, gate, fired);
 }
@@ -2497,8 +2500,9 @@ static void launch_stage2d_tile_k(const Ctx& c, const double* uc, const double* 
     const Geom& g = c.g;
     constexpr int bytes = (int)sizeof(TileShared<TY>);
     static std::atomic<unsigned long long> attr_set{0};
-    if (gk::first_on_device(attr_set))
+    gk::once_per_device(attr_set, [&] {
         cudaFuncSetAttribute(k_stage2d_tile<TY, KIND, PLM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    });
     const int tx = (g.nx + 27) / 28, tiles = tx * ((g.ny + TY - 1) / TY);
     const int grid = min(tiles, 148 * tile_ctas(TY));
     k_stage2d_tile<TY, KIND, PLM><<<grid, 32 * (TY + 2), bytes, s>>>(uc, u0, out, g, c.ph, c1, c2, c3, c.tm, tx);
@@ -2556,9 +2560,10 @@ static void launch_ens_stage_k(const gk::EnsInst* inst, const int4* tiles, int n
                                cudaStream_t s) {
     const size_t dyn = stage_dyn_bytes<NT, (KIND >= 1)>();
     static std::atomic<unsigned long long> attr_set{0};
-    if (gk::first_on_device(attr_set))
+    gk::once_per_device(attr_set, [&] {
         cudaFuncSetAttribute(k_ens_stage<NT, KIND, PLM>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    });
     k_ens_stage<NT, KIND, PLM><<<ctas, NT, dyn, s>>>(inst, tiles, ntiles, counter, c1, c2, c3);
 }
 

@@ -618,9 +618,10 @@ void launch_flux_correct(const float* model, const double* W, double* F, const G
                          const Phys& ph, const DevTime* tm, int dir, const FluxGate& gate,
                          unsigned* fired, cudaStream_t s) {
     static std::atomic<unsigned long long> attr{0};
-    if (gk::first_on_device(attr))
+    gk::once_per_device(attr, [&] {
         cudaFuncSetAttribute(k_flux_correct, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(InferShared));
+    });
     const long long nf = dir == 0 ? (long long)(g.nx + 1) * g.ny : (long long)g.nx * (g.ny + 1);
     const long long pairs = ((nf + 15) / 16 + 1) / 2;
     const int ctas = (int)((pairs + 3) / 4 < 148 * 8 ? (pairs + 3) / 4 : 148 * 8);
