@@ -20,6 +20,7 @@
 // 5 * vstride doubles fit (about 1290 x 1290 cells).
 #include <atomic>
 #include <cstdio>
+#include <cstring>
 #include <string>
 
 #include "gaukuk_cuda.h"
@@ -59,6 +60,14 @@ std::atomic<NoallocScratch*> g_scratch_addr[kMaxDevices];
 // (without reading cudaGetLastError, which would also report errors left by
 // unrelated work).
 std::atomic<unsigned long long> g_ticket{0};
+
+// The CFL reduction's start value, or the zero of a scratch that no call has used.
+bool is_seed(unsigned long long acc) {
+    const double seed = 1e-16;
+    unsigned long long bits;
+    std::memcpy(&bits, &seed, sizeof(bits));
+    return acc == bits || acc == 0;
+}
 
 }  // namespace
 
@@ -134,6 +143,14 @@ extern "C" int gk_rk2_step_noalloc(const gk_grid_desc* grid, const gk_phys_desc*
         cudaStreamSynchronize(s) != cudaSuccess)
         return GK_ERR_CUDA;
     const gk::DevTime& t = r.clock;
+    // The begin pass counts and reduces on from what the last call left, which is zero
+    // and the seed unless calls overlapped.  The last of those to copy its result sees
+    // what is left of them, and clears it for the calls that follow.
+    if (t.done_ctas || r.flag_acc || !is_seed(t.cmax_acc)) {
+        if (cudaMemsetAsync(&sc->res, 0, sizeof(sc->res), s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+            return GK_ERR_CUDA;
+    }
     if (r.ticket != ticket) {
         std::fprintf(stderr, "gk_rk2_step_noalloc: a kernel of this call did not launch\n");
         return GK_ERR_CUDA;
