@@ -63,6 +63,7 @@ SIGNATURES = {
     "gk_profile_steps": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_char_p, ctypes.c_int, _dp,
                                         _ip, ctypes.c_int, _ip]),
     "gk_fastmath_check": (ctypes.c_int, [ctypes.c_int, ctypes.c_ulonglong, _dp]),
+    "gk_fastmath_eval": (ctypes.c_int, [ctypes.c_int, _dp, _dp, _dp]),
     "gk_paritymath_eval": (ctypes.c_int, [ctypes.c_int, _dp, _dp, _dp]),
     "gk_checked_report": (ctypes.c_int, [ctypes.POINTER(ctypes.c_ulonglong),
                                          ctypes.POINTER(ctypes.c_ulonglong)]),

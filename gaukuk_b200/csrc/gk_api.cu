@@ -27,6 +27,7 @@
 
 namespace gk_fast {
 int fastmath_check(int n, unsigned long long seed, double* host_worst3);
+int math_eval(int n, const double* a, const double* b, double* out);
 }
 namespace gk_parity {
 int math_eval(int n, const double* a, const double* b, double* out);
@@ -1438,6 +1439,11 @@ int gk_checked_report(unsigned long long* count, unsigned long long* first) {
 int gk_fastmath_check(int n, unsigned long long seed, double* worst3) {
     if (n <= 0 || !worst3) return GK_ERR_INVALID;
     return gk_fast::fastmath_check(n, seed, worst3) == 0 ? GK_OK : GK_ERR_CUDA;
+}
+
+int gk_fastmath_eval(int n, const double* a, const double* b, double* out) {
+    if (n <= 0 || !a || !b || !out) return GK_ERR_INVALID;
+    return gk_fast::math_eval(n, a, b, out) == 0 ? GK_OK : GK_ERR_CUDA;
 }
 
 int gk_paritymath_eval(int n, const double* a, const double* b, double* out) {

@@ -47,4 +47,28 @@ int fastmath_check(int n, unsigned long long seed, double* host_worst3) {
     return e == cudaSuccess ? 0 : -1;
 }
 
+// The quotient and the root's products of n operand pairs (b positive):
+// out[0..n) = a/b, out[n..2n) = a/sqrt(b), out[2n..3n) = sqrt(b).
+__global__ void k_math_eval(int n, const double* __restrict__ a, const double* __restrict__ b,
+                            double* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        out[i] = div_nr(a[i], b[i]);
+        rsqrt_products(a[i], b[i], out[(size_t)n + i], out[2 * (size_t)n + i]);
+    }
+}
+
+int math_eval(int n, const double* a, const double* b, double* out) {
+    const size_t nb = sizeof(double) * (size_t)n;
+    double* d = nullptr;
+    if (cudaMalloc(&d, 5 * nb) != cudaSuccess) return -1;
+    cudaError_t e = cudaMemcpy(d, a, nb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, b, nb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_math_eval<<<148 * 4, 256>>>(n, d, d + n, d + 2 * (size_t)n);
+        e = cudaMemcpy(out, d + 2 * (size_t)n, 3 * nb, cudaMemcpyDeviceToHost);
+    }
+    cudaFree(d);
+    return e == cudaSuccess ? 0 : -1;
+}
+
 }  // namespace gk_fast

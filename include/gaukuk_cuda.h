@@ -352,6 +352,12 @@ int gk_tap_substeps(gk_handle* h, int nsub, double dt_sub, int ratio, double* fx
  * compiler's. */
 int gk_fastmath_check(int n, unsigned long long seed, double* worst3);
 
+/* Diagnostic of the FAST mode quotients and roots: a/b, a/sqrt(b) and sqrt(b) of n
+ * operand pairs with b > 0, as the kernels form them (host arrays; out holds 3n
+ * doubles).  Runs on the current device.  No counterpart in the reference, whose
+ * arithmetic is the host compiler's. */
+int gk_fastmath_eval(int n, const double* a, const double* b, double* out);
+
 /* Diagnostic of the PARITY mode arithmetic: its branch-free quotient a/b,
  * reciprocal 1/b and square root sqrt(a) of n operand pairs (host arrays; out
  * holds 3n doubles), which must equal the IEEE results for operands between
