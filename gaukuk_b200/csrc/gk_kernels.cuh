@@ -1,9 +1,8 @@
 // gk_kernels.cuh -- the device kernels of one arithmetic mode.
 //
-// Included by gk_kernels_parity.cu (GK_NS = gk_parity, GK_SEL = 0,
+// Included by gk_kernels_parity.cu (GK_NS = gk_parity, GK_FASTMATH = 0,
 // compiled with -fmad=false) and gk_kernels_fast.cu (GK_NS = gk_fast,
-// GK_SEL = 1, FMA contraction allowed); GK_SEL is the HLLC side selection
-// of gk_physics.cuh.
+// GK_FASTMATH = 1, FMA contraction allowed).
 //
 // Two implementations of one RK stage share the pointwise physics:
 //   * the generic path, one kernel per reference phase (ghost fill,
@@ -42,8 +41,6 @@ using gk::Ctx;
 using gk::DevTime;
 using gk::Geom;
 using gk::Phys;
-
-constexpr int kSel = GK_SEL;
 
 #ifndef GK_CHECKED
 #define GK_CHECKED 0
@@ -371,7 +368,7 @@ __global__ void k_flux(const double* __restrict__ w, double* __restrict__ F, Geo
     const int s1 = dir == 0 ? gk::P_VY : (dir == 1 ? gk::P_VZ : gk::P_VX);
     const int s2 = dir == 0 ? gk::P_VZ : (dir == 1 ? gk::P_VX : gk::P_VY);
     Flux5 f;
-    hllc<true, kSel>(wl[gk::P_RHO], wl[sn], wl[s1], wl[s2], wl[gk::P_PRE], wr[gk::P_RHO], wr[sn],
+    hllc<true>(wl[gk::P_RHO], wl[sn], wl[s1], wl[s2], wl[gk::P_PRE], wr[gk::P_RHO], wr[sn],
                      wr[s1], wr[s2], wr[gk::P_PRE], ph, f);
     // momentum slots of the rotated components (slot ids equal prim ids)
     const long long c = fidx(g, k, j, i);
@@ -970,7 +967,7 @@ __global__ void __launch_bounds__(NT, 1)
 #pragma unroll
             for (int v = 0; v < 5; ++v) s[v] = sm.XL[v][l - 1];
             Flux5 f;
-            hllc<true, kSel>(s[gk::P_RHO], s[gk::P_VX], s[gk::P_VY], s[gk::P_VZ], s[gk::P_PRE],
+            hllc<true>(s[gk::P_RHO], s[gk::P_VX], s[gk::P_VY], s[gk::P_VZ], s[gk::P_PRE],
                              xr[gk::P_RHO], xr[gk::P_VX], xr[gk::P_VY], xr[gk::P_VZ], xr[gk::P_PRE],
                              ph, f);
             fx[gk::S_DEN] = f.d;
@@ -1186,7 +1183,7 @@ __device__ __forceinline__ Q4 ldq(const double* __restrict__ u, long long vs, lo
 
 // y face: rotation (vy | vz, vx) with vz = 0, so tangential 1 carries vx.
 __device__ __forceinline__ void hllc_y(const W4& l, const W4& r, const Phys& ph, Flux5& f) {
-    hllc<false, kSel>(l.r, l.vy, l.vx, 0.0, l.p, r.r, r.vy, r.vx, 0.0, r.p, ph, f);
+    hllc<false>(l.r, l.vy, l.vx, 0.0, l.p, r.r, r.vy, r.vx, 0.0, r.p, ph, f);
 }
 // The x face (rotation (vx | vy, vz)) and the y face of a row, solved
 // together: both Riemann problems are straight-line code, so their
@@ -1196,15 +1193,15 @@ __device__ __forceinline__ void hllc_xy(const W4& xl, const W4& xr, Flux5& fx, c
                                         const W4& yr, Flux5& fy, const Phys& ph) {
     bool badx = !ph.ranged, bady = !ph.ranged;
     HllcAux ax, ay;
-    hllc_ranged<false, kSel>(xl.r, xl.vx, xl.vy, 0.0, xl.p, xr.r, xr.vx, xr.vy, 0.0, xr.p, ph, fx,
+    hllc_ranged<false>(xl.r, xl.vx, xl.vy, 0.0, xl.p, xr.r, xr.vx, xr.vy, 0.0, xr.p, ph, fx,
                              badx, ax);
-    hllc_ranged<false, kSel>(yl.r, yl.vy, yl.vx, 0.0, yl.p, yr.r, yr.vy, yr.vx, 0.0, yr.p, ph, fy,
+    hllc_ranged<false>(yl.r, yl.vy, yl.vx, 0.0, yl.p, yr.r, yr.vy, yr.vx, 0.0, yr.p, ph, fy,
                              bady, ay);
 #if !GK_FASTMATH
     if (badx || bady || ax.zero || ay.zero) {
-        hllc_redo<false, kSel>(xl.r, xl.vx, xl.vy, 0.0, xl.p, xr.r, xr.vx, xr.vy, 0.0, xr.p, ph, fx,
+        hllc_redo<false>(xl.r, xl.vx, xl.vy, 0.0, xl.p, xr.r, xr.vx, xr.vy, 0.0, xr.p, ph, fx,
                                badx, ax);
-        hllc_redo<false, kSel>(yl.r, yl.vy, yl.vx, 0.0, yl.p, yr.r, yr.vy, yr.vx, 0.0, yr.p, ph, fy,
+        hllc_redo<false>(yl.r, yl.vy, yl.vx, 0.0, yl.p, yr.r, yr.vy, yr.vx, 0.0, yr.p, ph, fy,
                                bady, ay);
     }
 #endif
@@ -1803,9 +1800,6 @@ __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CU
     constexpr int RD = 4 * NT;
     constexpr unsigned RB = RD * sizeof(double);
     unsigned long long cbest = 0ull;
-#if !GK_FASTMATH
-    const bool unit = !THREE && c1 == 1.0 && c2 == 1.0;
-#endif
 
     const double dt = tm->dt;
     const double dtdx = dt * g.dxRec, dtdy = dt * g.dyRec;
@@ -1994,17 +1988,11 @@ __device__ __forceinline__ void stage_tile_tma(const CUtensorMap* mapc, const CU
                 r[1] = c1 * U0.mx + c2 * Qm1.mx - c3 * dF1;
                 r[2] = c1 * U0.my + c2 * Qm1.my - c3 * dF2;
                 r[3] = c1 * U0.e + c2 * Qm1.e - c3 * dF3;
-            } else if (unit) {
-                // c1 = c2 = 1 (every integrator's first stage): the products are exact
+            } else {  // a first stage: c1 = c2 = 1
                 r[0] = Qm1.d - dF0;
                 r[1] = Qm1.mx - dF1;
                 r[2] = Qm1.my - dF2;
                 r[3] = Qm1.e - dF3;
-            } else {
-                r[0] = c1 * Qm1.d - c2 * dF0;
-                r[1] = c1 * Qm1.mx - c2 * dF1;
-                r[2] = c1 * Qm1.my - c2 * dF2;
-                r[3] = c1 * Qm1.e - c2 * dF3;
             }
 #endif
             double press;

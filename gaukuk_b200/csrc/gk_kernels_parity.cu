@@ -1,7 +1,6 @@
 // Kernels in parity mode: compiled with -fmad=false, correctly rounded
 // division and square root, the reference's bits (gk_physics.cuh).
 #define GK_NS gk_parity
-#define GK_SEL 0
 #define GK_FASTMATH 0
 #include "gk_kernels.cuh"
 

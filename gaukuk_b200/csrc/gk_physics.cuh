@@ -105,10 +105,6 @@ __device__ __forceinline__ double floor_at(double x, double f) {
 #define GK_RCP(b) rcp_any(b)
 #define GK_SQRT(x) sqrt_any(x)
 // the reference's compares and std::max/min
-#define GK_MAX0(x) smax((x), 0.0)
-#define GK_MIN0(x) smin(0.0, (x))
-#define GK_GE0(x) ((x) >= 0)
-#define GK_LE0(x) ((x) <= 0.0)
 #define GK_FLOOR(x, f) smax((x), (f))
 #define GK_BELOW(x, f) ((x) < (f))
 #define GK_MAXNN(a, b) smax((a), (b))
@@ -239,17 +235,6 @@ __device__ __forceinline__ double sqrt_any(double x) {
 }
 #endif
 
-// Reconstruction::VanLeer (reconstruction.hpp:36-42).
-__device__ __forceinline__ double vanleer(double a, double b) {
-    double multi = a * b;
-#if GK_FASTMATH
-    double sigma = GK_DIV(2.0 * multi, a + b);
-    return (multi <= 0.0) ? 0.0 : sigma;
-#else
-    return (multi <= 0.0) ? 0.0 : GK_DIV(2.0 * multi, a + b);
-#endif
-}
-
 // Half the van Leer slope: what the PLM face states u +- 0.5*sigma add.  Fast
 // mode: (a*b)/(a+b) for ab > 0 else 0, without the two scalings by 2 and 1/2.
 // Parity mode: the same quotient, which is exactly 0.5*((2ab)/(a+b)) unless a
@@ -291,7 +276,11 @@ __device__ __forceinline__ double vanleer_half(double a, double b, SlopeRange& r
     const double h = div_rn_plain(multi, sum);
     return none ? 0.0 : h;
 }
-__device__ __noinline__ double vanleer_half_any(double a, double b) { return 0.5 * vanleer(a, b); }
+// Half of Reconstruction::VanLeer (reconstruction.hpp:36-42).
+__device__ __noinline__ double vanleer_half_any(double a, double b) {
+    const double multi = a * b;
+    return 0.5 * ((multi <= 0.0) ? 0.0 : GK_DIV(2.0 * multi, a + b));
+}
 #endif
 
 struct Flux5 {
@@ -305,28 +294,21 @@ struct Flux5 {
 // tangential component, which callers use only when it is exactly zero (2D
 // runs with vz = 0): every term it contributes is then an exact zero.
 //
-// SEL picks how the two star sides are combined, f = selectl*fl + selectr*fr
-// with selectl = (ss >= 0) ? 1 : 0 (hllc.cpp:75-94): 0 both sides, as the
-// reference writes it (parity mode); 1 only the selected side (fast mode),
-// which differs only where the unused side is not finite, or in the sign of
-// a zero.
-template <bool T2, int SEL>
+// The reference combines its star sides as f = selectl*fl + selectr*fr with
+// selectl = (ss >= 0) ? 1 : 0 (hllc.cpp:75-94), and so does parity mode here; fast
+// mode evaluates the selected side only, which differs where the unused side is
+// not finite, or in the sign of a zero.
+#if GK_FASTMATH
+template <bool T2>
 __device__ __forceinline__ void hllc_any(double denl, double vxl, double vyl, double vzl, double prel,
                                          double denr, double vxr, double vyr, double vzr, double prer,
                                          const gk::Phys& ph, Flux5& f) {
     const double gamma = ph.gamma;
-#if GK_FASTMATH
     // sqrt(gamma*p/rho) = (gamma*p) * rsqrt(gamma*p*rho): one root, no quotient
     const double gpl = gamma * prel, gpr = gamma * prer;
     double al, ar, unused;
     rsqrt_products(gpl, gpl * denl, al, unused);
     rsqrt_products(gpr, gpr * denr, ar, unused);
-#else
-    // EquationOfState::SoundSpeed (eos.hpp:27-29)
-    double al = sqrt(GK_DIV(gamma * prel, denl));
-    double ar = sqrt(GK_DIV(gamma * prer, denr));
-#endif
-#if GK_FASTMATH
     // 2p* of the PVRS estimate; max(p*, 0) is not taken, as only max(p* - p, 0)
     // of positive pressures p is used
     const double pvrs2 = fma(-0.25 * ((vxr - vxl) * (denl + denr)), al + ar, prel + prer);
@@ -344,9 +326,42 @@ __device__ __forceinline__ void hllc_any(double denl, double vxl, double vyl, do
     ml = -ml;
     double sl = vxl - dvl;
     double sr = vxr + dvr;
+    // the contact speed's numerator and (negative) denominator, with rho (S - v)
+    // of each side formed once
+    const double num = prer - prel + ml * vxl - mr * vxr, den = ml - mr;
+    double ss = GK_DIV(num, den);
+    // The selected side: its kinetic energy from the selected velocities, and
+    // E + p as p/(gamma-1) + p + rho k/2 in one product with gamma/(gamma-1).
+    // m = rho (S - v) of the side, formed for the contact speed, carries the
+    // star-state terms:
+    //   rho (vn^2 + c S) = f1 vn + c m,   rho c ss (S - vn) = c ss m.
+    const bool left = GK_LE0(num);
+    double d = left ? denl : denr, vn = left ? vxl : vxr, v1 = left ? vyl : vyr;
+    double v2 = left ? vzl : vzr, p = left ? prel : prer, s = left ? sl : sr;
+    const double m = left ? ml : mr;
+    double k = T2 ? (vn * vn + v1 * v1 + v2 * v2) : (vn * vn + v1 * v1);
+    double ep = p * ph.gm1Rec1 + 0.5 * d * k;  // E + p
+    double sc = left ? GK_MIN0(s) : GK_MAX0(s);
+    double c = GK_DIV(sc * (ss - vn), s - ss);
+    double vc = vn + c;
+    double f1 = d * vc;
+    f.d = f1;
+    f.n = f1 * vn + (c * m + p);
+    f.t1 = f1 * v1;
+    f.t2 = T2 ? f1 * v2 : 0.0;
+    f.e = ep * vc + c * ss * m;
+}
 #else
+template <bool T2>
+__device__ __forceinline__ void hllc_any(double denl, double vxl, double vyl, double vzl, double prel,
+                                         double denr, double vxr, double vyr, double vzr, double prer,
+                                         const gk::Phys& ph, Flux5& f) {
+    const double gamma = ph.gamma;
+    // EquationOfState::SoundSpeed (eos.hpp:27-29)
+    double al = sqrt(GK_DIV(gamma * prel, denl));
+    double ar = sqrt(GK_DIV(gamma * prer, denr));
     double prePVRS = 0.5 * (prel + prer) - 0.125 * (vxr - vxl) * (denl + denr) * (al + ar);
-    prePVRS = GK_MAX0(prePVRS);
+    prePVRS = smax(prePVRS, 0.0);
     double ql, qr;
     // q = sqrt(1 + 0.5*(1+1/gamma)*max(p*/p - 1, 0)) is exactly 1 whenever
     // p* <= p with p > 0, so the division and root are skipped there.
@@ -362,91 +377,50 @@ __device__ __forceinline__ void hllc_any(double denl, double vxl, double vyl, do
     }
     double sl = vxl - al * ql;
     double sr = vxr + ar * qr;
-#endif
-#if GK_FASTMATH
-    // the contact speed's numerator and (negative) denominator, with rho (S - v)
-    // of each side formed once
-    const double num = prer - prel + ml * vxl - mr * vxr, den = ml - mr;
-    double ss = GK_DIV(num, den);
-#else
     double ss = GK_DIV(prer - prel + denl * vxl * (sl - vxl) - denr * vxr * (sr - vxr),
                        denl * (sl - vxl) - denr * (sr - vxr));
-#endif
-    auto both_sides = [&]() {
-        // EquationOfState::EGas (eos.hpp:30-32) + kinetic energy
-        double kl = T2 ? (vxl * vxl + vyl * vyl + vzl * vzl) : (vxl * vxl + vyl * vyl);
-        double kr = T2 ? (vxr * vxr + vyr * vyr + vzr * vzr) : (vxr * vxr + vyr * vyr);
-        double el = prel * ph.gm1Rec + 0.5 * denl * kl;
-        double er = prer * ph.gm1Rec + 0.5 * denr * kr;
-        double cl = GK_DIV(smin(0.0, sl) * (ss - vxl), sl - ss);
-        double cr = GK_DIV(smax(0.0, sr) * (ss - vxr), sr - ss);
-        double selectl = (ss >= 0) ? 1.0 : 0.0;
-        double selectr = 1.0 - selectl;
-        double fl1 = denl * (vxl + cl);
-        double fl2 = denl * (vxl * vxl + cl * sl) + prel;
-        double fl3 = fl1 * vyl;
-        double fl5 = (el + prel) * (vxl + cl) + denl * cl * ss * (sl - vxl);
-        double fr1 = denr * (vxr + cr);
-        double fr2 = denr * (vxr * vxr + cr * sr) + prer;
-        double fr3 = fr1 * vyr;
-        double fr5 = (er + prer) * (vxr + cr) + denr * cr * ss * (sr - vxr);
-        f.d = selectl * fl1 + selectr * fr1;
-        f.n = selectl * fl2 + selectr * fr2;
-        f.t1 = selectl * fl3 + selectr * fr3;
-        if (T2) {
-            double fl4 = fl1 * vzl;
-            double fr4 = fr1 * vzr;
-            f.t2 = selectl * fl4 + selectr * fr4;
-        } else {
-            f.t2 = 0.0;
-        }
-        f.e = selectl * fl5 + selectr * fr5;
-    };
-    if (SEL == 0) {
-        both_sides();
-        return;
+    // EquationOfState::EGas (eos.hpp:30-32) + kinetic energy
+    double kl = T2 ? (vxl * vxl + vyl * vyl + vzl * vzl) : (vxl * vxl + vyl * vyl);
+    double kr = T2 ? (vxr * vxr + vyr * vyr + vzr * vzr) : (vxr * vxr + vyr * vyr);
+    double el = prel * ph.gm1Rec + 0.5 * denl * kl;
+    double er = prer * ph.gm1Rec + 0.5 * denr * kr;
+    double cl = GK_DIV(smin(0.0, sl) * (ss - vxl), sl - ss);
+    double cr = GK_DIV(smax(0.0, sr) * (ss - vxr), sr - ss);
+    double selectl = (ss >= 0) ? 1.0 : 0.0;
+    double selectr = 1.0 - selectl;
+    double fl1 = denl * (vxl + cl);
+    double fl2 = denl * (vxl * vxl + cl * sl) + prel;
+    double fl3 = fl1 * vyl;
+    double fl5 = (el + prel) * (vxl + cl) + denl * cl * ss * (sl - vxl);
+    double fr1 = denr * (vxr + cr);
+    double fr2 = denr * (vxr * vxr + cr * sr) + prer;
+    double fr3 = fr1 * vyr;
+    double fr5 = (er + prer) * (vxr + cr) + denr * cr * ss * (sr - vxr);
+    f.d = selectl * fl1 + selectr * fr1;
+    f.n = selectl * fl2 + selectr * fr2;
+    f.t1 = selectl * fl3 + selectr * fr3;
+    if (T2) {
+        double fl4 = fl1 * vzl;
+        double fr4 = fr1 * vzr;
+        f.t2 = selectl * fl4 + selectr * fr4;
+    } else {
+        f.t2 = 0.0;
     }
-    // The selected side only (fast mode): its kinetic energy from the
-    // selected velocities, and E + p as p/(gamma-1) + p + rho k/2 in one
-    // product with gamma/(gamma-1).  m = rho (S - v) of the side, formed for
-    // the contact speed, carries the star-state terms:
-    //   rho (vn^2 + c S) = f1 vn + c m,   rho c ss (S - vn) = c ss m.
-#if GK_FASTMATH
-    const bool left = GK_LE0(num);
-#else
-    const bool left = GK_GE0(ss);
-#endif
-    double d = left ? denl : denr, vn = left ? vxl : vxr, v1 = left ? vyl : vyr;
-    double v2 = left ? vzl : vzr, p = left ? prel : prer, s = left ? sl : sr;
-#if GK_FASTMATH
-    const double m = left ? ml : mr;
-#else
-    const double m = d * (s - vn);  // unused: parity mode evaluates both sides
-#endif
-    double k = T2 ? (vn * vn + v1 * v1 + v2 * v2) : (vn * vn + v1 * v1);
-    double ep = p * ph.gm1Rec1 + 0.5 * d * k;  // E + p
-    double sc = left ? GK_MIN0(s) : GK_MAX0(s);
-    double c = GK_DIV(sc * (ss - vn), s - ss);
-    double vc = vn + c;
-    double f1 = d * vc;
-    f.d = f1;
-    f.n = f1 * vn + (c * m + p);
-    f.t1 = f1 * v1;
-    f.t2 = T2 ? f1 * v2 : 0.0;
-    f.e = ep * vc + c * ss * m;
+    f.e = selectl * fl5 + selectr * fr5;
 }
+#endif
 
 #if GK_FASTMATH
 // Fast mode has one form: no lane is ever out of its range.
 struct HllcAux {};
-template <bool T2, int SEL>
+template <bool T2>
 __device__ __forceinline__ void hllc_ranged(double denl, double vxl, double vyl, double vzl,
                                             double prel, double denr, double vxr, double vyr,
                                             double vzr, double prer, const gk::Phys& ph, Flux5& f,
                                             bool&, HllcAux&) {
-    hllc_any<T2, SEL>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f);
+    hllc_any<T2>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f);
 }
-template <bool T2, int SEL>
+template <bool T2>
 __device__ __forceinline__ void hllc_redo(double, double, double, double, double, double, double,
                                           double, double, double, const gk::Phys&, Flux5&, bool,
                                           const HllcAux&) {}
@@ -461,7 +435,7 @@ struct HllcAux {
     double ss, so;  // contact speed, the other side's wave speed
     bool zero;      // a component of the selected side is -0
 };
-template <bool T2, int SEL>
+template <bool T2>
 __device__ __forceinline__ void hllc_ranged(double denl, double vxl, double vyl, double vzl,
                                             double prel, double denr, double vxr, double vyr,
                                             double vzr, double prer, const gk::Phys& ph, Flux5& f,
@@ -523,14 +497,14 @@ __device__ __forceinline__ void hllc_ranged(double denl, double vxl, double vyl,
 struct HllcStates {
     double denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer;
 };
-template <bool T2, int SEL>
+template <bool T2>
 __device__ __noinline__ Flux5 hllc_far(HllcStates w, double gamma, double gm1Rec, double cq) {
     gk::Phys ph;
     ph.gamma = gamma;
     ph.gm1Rec = gm1Rec;
     ph.cq = cq;
     Flux5 f;
-    hllc_any<T2, SEL>(w.denl, w.vxl, w.vyl, w.vzl, w.prel, w.denr, w.vxr, w.vyr, w.vzr, w.prer, ph, f);
+    hllc_any<T2>(w.denl, w.vxl, w.vyl, w.vzl, w.prel, w.denr, w.vxr, w.vyr, w.vzr, w.prer, ph, f);
     return f;
 }
 
@@ -539,7 +513,7 @@ __device__ __noinline__ Flux5 hllc_far(HllcStates w, double gamma, double gm1Rec
 // the seed reciprocal (relative error 2^-19): unless v and c cancel to 2^-16,
 // that sign is certain.  The momenta's signs follow from it; a -0 energy flux
 // and a cancellation take the full evaluation.
-template <bool T2, int SEL>
+template <bool T2>
 __device__ __forceinline__ void hllc_redo(double denl, double vxl, double vyl, double vzl,
                                           double prel, double denr, double vxr, double vyr,
                                           double vzr, double prer, const gk::Phys& ph, Flux5& f,
@@ -566,21 +540,21 @@ __device__ __forceinline__ void hllc_redo(double denl, double vxl, double vyl, d
         if (T2) zero(f.t2, neg ^ hi(v2));
     }
     if (bad)
-        f = hllc_far<T2, SEL>(HllcStates{denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer},
+        f = hllc_far<T2>(HllcStates{denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer},
                               ph.gamma, ph.gm1Rec, ph.cq);
 }
 #endif
 
 // Flux::RiemannSolver for one face of any state.
-template <bool T2, int SEL>
+template <bool T2>
 __device__ __forceinline__ void hllc(double denl, double vxl, double vyl, double vzl, double prel,
                                      double denr, double vxr, double vyr, double vzr, double prer,
                                      const gk::Phys& ph, Flux5& f) {
     bool bad = !ph.ranged;
     HllcAux aux;
-    hllc_ranged<T2, SEL>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f, bad, aux);
+    hllc_ranged<T2>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f, bad, aux);
 #if !GK_FASTMATH
     if (bad || aux.zero)
-        hllc_redo<T2, SEL>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f, bad, aux);
+        hllc_redo<T2>(denl, vxl, vyl, vzl, prel, denr, vxr, vyr, vzr, prer, ph, f, bad, aux);
 #endif
 }

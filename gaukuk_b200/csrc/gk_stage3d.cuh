@@ -70,7 +70,7 @@ __device__ __forceinline__ void slots_y(const Flux5& f, double (&F)[5]) {
 __device__ __forceinline__ void hllc5_y(const double (&l)[5], const double (&r)[5], const Phys& ph,
                                         double (&F)[5]) {
     Flux5 f;
-    hllc<true, kSel>(l[gk::P_RHO], l[gk::P_VY], l[gk::P_VZ], l[gk::P_VX], l[gk::P_PRE], r[gk::P_RHO],
+    hllc<true>(l[gk::P_RHO], l[gk::P_VY], l[gk::P_VZ], l[gk::P_VX], l[gk::P_PRE], r[gk::P_RHO],
                      r[gk::P_VY], r[gk::P_VZ], r[gk::P_VX], r[gk::P_PRE], ph, f);
     slots_y(f, F);
 }
@@ -84,12 +84,12 @@ __device__ __forceinline__ void hllc5_xy(const double (&xl)[5], const double (&x
                  xr[gk::P_RHO], xr[gk::P_VX], xr[gk::P_VY], xr[gk::P_VZ], xr[gk::P_PRE], ph, fx, badx, ax
 #define GK_YARGS yl[gk::P_RHO], yl[gk::P_VY], yl[gk::P_VZ], yl[gk::P_VX], yl[gk::P_PRE], \
                  yr[gk::P_RHO], yr[gk::P_VY], yr[gk::P_VZ], yr[gk::P_VX], yr[gk::P_PRE], ph, fy, bady, ay
-    hllc_ranged<true, kSel>(GK_XARGS);
-    hllc_ranged<true, kSel>(GK_YARGS);
+    hllc_ranged<true>(GK_XARGS);
+    hllc_ranged<true>(GK_YARGS);
 #if !GK_FASTMATH
     if (badx || bady || ax.zero || ay.zero) {
-        hllc_redo<true, kSel>(GK_XARGS);
-        hllc_redo<true, kSel>(GK_YARGS);
+        hllc_redo<true>(GK_XARGS);
+        hllc_redo<true>(GK_YARGS);
     }
 #endif
 #undef GK_XARGS
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(128)
         if (mine) {
             // z face (k-1 | k): (vz | vx, vy)
             Flux5 f;
-            hllc<true, kSel>(wl[gk::P_RHO], wl[gk::P_VZ], wl[gk::P_VX], wl[gk::P_VY],
+            hllc<true>(wl[gk::P_RHO], wl[gk::P_VZ], wl[gk::P_VX], wl[gk::P_VY],
                              wl[gk::P_PRE], wr[gk::P_RHO], wr[gk::P_VZ], wr[gk::P_VX],
                              wr[gk::P_VY], wr[gk::P_PRE], ph, f);
             double fz[5];
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kRowThreads, CTAS)
         }
         __syncthreads();
         Flux5 f;
-        hllc<true, kSel>(sXL[gk::P_RHO][tl], sXL[gk::P_VX][tl], sXL[gk::P_VY][tl],
+        hllc<true>(sXL[gk::P_RHO][tl], sXL[gk::P_VX][tl], sXL[gk::P_VY][tl],
                          sXL[gk::P_VZ][tl], sXL[gk::P_PRE][tl], xr[gk::P_RHO], xr[gk::P_VX],
                          xr[gk::P_VY], xr[gk::P_VZ], xr[gk::P_PRE], ph, f);
         double fx[5];
