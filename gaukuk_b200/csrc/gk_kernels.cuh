@@ -1207,6 +1207,39 @@ __device__ __forceinline__ void hllc_xy(const W4& xl, const W4& xr, Flux5& fx, c
 #endif
 }
 
+// The end of a step's last stage: the CTA's largest CFL speed (bit pattern)
+// into the clock; the last of `ctas` CTAs runs the step epilogue (a slab of a
+// split grid leaves that to launch_epilogue, after the maximum over all slabs).
+template <int NT>
+__device__ __forceinline__ void last_stage_end(unsigned long long cbest, DevTime* tm, const Geom& g,
+                                               const Phys& ph, unsigned ctas) {
+    __shared__ unsigned long long wmax[NT / 32];
+    __shared__ int last;
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, cbest, o);
+        cbest = x > cbest ? x : cbest;
+    }
+    if ((t & 31) == 0) wmax[t >> 5] = cbest;
+    __syncthreads();
+    if (t == 0) {
+        unsigned long long m = wmax[0];
+        for (int w = 1; w < NT / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
+        atomicMax(&tm->cmax_acc, m);
+        last = 0;
+        if (!ph.defer_epilogue) {
+            __threadfence();
+            last = atomicAdd(&tm->done_ctas, 1u) == ctas - 1;
+        }
+    }
+    __syncthreads();
+    if (last && t == 0) {
+        __threadfence();
+        step_epilogue(tm, g, ph, 1);
+    }
+}
+
 // KIND 0: u' = c1*uc - c2*dF (stage 1); 1: u' = c1*u0 + c2*uc - c3*dF
 // (later stages); 2: as 1 and the last stage of the step, which also applies
 // the gravity half kick (sim.cpp:89-91), reduces the CFL speed of the new
@@ -1358,63 +1391,7 @@ __global__ void __launch_bounds__(kStageThreads, 3)
         Qm1 = Q0;
         Q0 = Q1;
     }
-    if (LAST) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long x = __shfl_xor_sync(0xffffffffu, cbest, o);
-            cbest = x > cbest ? x : cbest;
-        }
-        __shared__ unsigned long long wmax[kStageThreads / 32];
-        __shared__ bool last;
-        if ((t & 31) == 0) wmax[t >> 5] = cbest;
-        __syncthreads();
-        if (t == 0) {
-            unsigned long long m = wmax[0];
-            for (int w = 1; w < kStageThreads / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
-            atomicMax(&tm->cmax_acc, m);
-            __threadfence();
-            const unsigned int prev = atomicAdd(&tm->done_ctas, 1u);
-            last = (prev == gridDim.x * gridDim.y - 1);
-        }
-        __syncthreads();
-        if (last && t == 0) {
-            __threadfence();
-            step_epilogue(tm, g, ph, 1);
-        }
-    }
-}
-
-// The end of a step's last stage: the CTA's largest CFL speed (bit pattern)
-// into the clock; the last of `ctas` CTAs runs the step epilogue (a slab of a
-// split grid leaves that to launch_epilogue, after the maximum over all slabs).
-template <int NT>
-__device__ __forceinline__ void last_stage_end(unsigned long long cbest, DevTime* tm, const Geom& g,
-                                               const Phys& ph, unsigned ctas) {
-    __shared__ unsigned long long wmax[NT / 32];
-    __shared__ int last;
-    const int t = threadIdx.x;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long x = __shfl_xor_sync(0xffffffffu, cbest, o);
-        cbest = x > cbest ? x : cbest;
-    }
-    if ((t & 31) == 0) wmax[t >> 5] = cbest;
-    __syncthreads();
-    if (t == 0) {
-        unsigned long long m = wmax[0];
-        for (int w = 1; w < NT / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
-        atomicMax(&tm->cmax_acc, m);
-        last = 0;
-        if (!ph.defer_epilogue) {
-            __threadfence();
-            last = atomicAdd(&tm->done_ctas, 1u) == ctas - 1;
-        }
-    }
-    __syncthreads();
-    if (last && t == 0) {
-        __threadfence();
-        step_epilogue(tm, g, ph, 1);
-    }
+    if (LAST) last_stage_end<kStageThreads>(cbest, tm, g, ph, gridDim.x * gridDim.y);
 }
 
 // ------------------------------------------------------------ fused 2D stage, small grids
