@@ -159,6 +159,7 @@ struct gk_handle {
     cudaGraphExec_t gexec = nullptr;
     int graph_steps = 0;
     int graph_path = -1;
+    bool fixed_vz = false;  // 1D/2D: the fixed data hold a z momentum
     // sides whose ghost fill is a host routine (gk_set_host_fill)
     struct HostFill {
         int side, depth;
@@ -901,10 +902,14 @@ bool host_all_zero(const double* p, size_t n) {
     return true;
 }
 
-// Whether a 1D or 2D run makes a z momentum that is zero at upload non-zero: a
+// Whether a 1D or 2D run may make a z momentum that is zero at upload non-zero: a
 // point mass off the mid-plane and z gravity do, an immersed body writes it
-// (signed zeros in 2D) into its shell cells.
-bool makes_vz(const gk::Phys& ph) { return ph.npoint || ph.nshell || ph.grav[2] != 0; }
+// (signed zeros in 2D) into its shell cells, fixed data may hold some and a host
+// routine may write it.
+bool makes_vz(const gk_handle* h) {
+    const gk::Phys& ph = h->ctx.ph;
+    return ph.npoint || ph.nshell || ph.grav[2] != 0 || h->fixed_vz || !h->host_fills.empty();
+}
 
 // The captured graph holds launches that no longer fit: rebuilt at the next one.
 void drop_graph(gk_handle* h) {
@@ -922,7 +927,7 @@ std::array<int, 6> upload_choices(const gk::Ctx& c) {
 // A change of the physics that kernels take by value: the captured graph
 // is rebuilt at the next launch, and the path follows.
 int physics_changed(gk_handle* h) {
-    if (makes_vz(h->ctx.ph)) h->ctx.has_vz = 1;
+    if (makes_vz(h)) h->ctx.has_vz = 1;
     drop_graph(h);
     if (h->uploaded) {
         set_path(h);
@@ -1059,7 +1064,7 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
         GK_CUDA(h, cudaStreamSynchronize(h->stream));
         h->ctx.has_vz = flag;
     }
-    if (makes_vz(h->ctx.ph)) h->ctx.has_vz = 1;
+    if (makes_vz(h)) h->ctx.has_vz = 1;
     set_path(h);
     h->ctx.use_tma = env_int("GK_STAGE_TMA", 1) != 0;
     if (!h->tiling_set) {
@@ -1936,6 +1941,7 @@ extern "C" int gk_set_fixed_boundary(gk_handle* h, const double* snapshot, int f
     if (!snapshot) {
         ph.fixed_bd = nullptr;
         ph.fix_inner = 0;
+        h->fixed_vz = false;
         return physics_changed(h);
     }
     if (!h->fixed) {
@@ -1945,6 +1951,8 @@ extern "C" int gk_set_fixed_boundary(gk_handle* h, const double* snapshot, int f
     }
     int rc = copy_ref_to_device(h, snapshot, h->fixed);
     if (rc != GK_OK) return rc;
+    const size_t plane = (size_t)g.lenx * g.leny;
+    h->fixed_vz = g.ndim <= 2 && !host_all_zero(snapshot + (3 * (size_t)g.lenz + g.kofs) * plane, plane);
     GK_CUDA(h, cudaStreamSynchronize(h->stream));
     ph.fixed_bd = h->fixed;
     ph.fix_inner = fix_inner ? 1 : 0;
