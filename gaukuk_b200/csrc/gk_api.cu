@@ -153,6 +153,7 @@ struct gk_handle {
     gk::Shell* shells = nullptr;  // immersed body's shell table (device)
     int shell_cap = 0;
     bool mtz_plane_zero = false;  // 1D/2D: every stored MTZ value was +0.0 at upload
+    bool mtz_stepped = false;     // a path that writes MTZ has run: B and C may hold one
     long long io_up = 0, io_down = 0;  // bytes the last upload / download moved
     unsigned* fired = nullptr;  // faces where the detector kept plain HLLC
     int tiling_rows = 0;
@@ -753,6 +754,7 @@ int pull_time(gk_handle* h) {
 // or the output time may have ended the run) decides whose strips are kept if
 // the new ones do not run: that is read from the clock, once per change.
 int note_steps(gk_handle* h, const double* buf) {
+    h->mtz_stepped = h->mtz_stepped || h->path != 1;
     if (buf == h->strips_next) return GK_OK;
     if (h->strips_next) {
         const int rc = pull_time(h);
@@ -1078,6 +1080,16 @@ int gk_upload_cons(gk_handle* h, const double* cons) {
         h->ctx.learn_rows = 0;
     }
     if (upload_choices(h->ctx) != before) drop_graph(h);
+    // What an earlier state's steps left in the stage buffers and the new one's steps
+    // will not write: the z momentum off the five-variable paths, whose ghosts a frame
+    // shows, and the ghosts that a one-cell grid's fill copies.
+    if (h->mtz_stepped && (h->path == 1 || g.nx == 1)) {
+        const size_t from = g.nx == 1 ? 0 : gk::S_MTZ * (size_t)g.vstride;
+        const size_t bytes = sizeof(double) * (5 * (size_t)g.vstride - from);
+        for (double* p : {h->B, h->C})
+            if (p) GK_CUDA(h, cudaMemsetAsync(p + from, 0, bytes, h->stream));
+        h->mtz_stepped = false;
+    }
     if (h->path != 1) {
         int rc = alloc_generic(h);
         if (rc != GK_OK) return rc;
