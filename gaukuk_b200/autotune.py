@@ -5,7 +5,9 @@ threads updates T-4 columns and marches up R rows.  Narrow, short tiles give
 more CTAs (better for small grids), wide, long ones less halo work.  The
 tuner measures rather than models: it times a few device-resident steps for
 each candidate with CUDA events on the library's stream and keeps the
-fastest.
+fastest.  Grids small enough for the tile form of the stage (28 columns x 4 or
+10 rows, chosen by itself; gk_set_tiling turns it off) are usually faster
+untuned.
 
 * ``tune_single(sim)``: one problem; sets the winner with gk_set_tiling.
 * ``tune_ensemble(ens)``: threads first (one value for the whole persistent

@@ -420,8 +420,9 @@ int stage_rows(const gk::Geom& g, int threads, bool parity) {
 //   22.5];
 //   marching, one wave of r rows filling a share L of the slots: 3 + (r + 1.4)
 //   (4.2 + 2.1 L) / 3 + (r + 1.4)(2.9 + 2.0 L) [512^2, r = 6 / 4: 45.3 / 27.9].
-// Tiles are taken where they save at least 9 % by it, so that a grid whose tiles
-// are partly empty does not lose (1000x60: 19.5 / 14.6 either way).
+// Tiles of 4 rows are taken wherever each has a resident slot (two per SM), which
+// needs no model; tiles of 10 where they save at least 9 % by it, so that a grid
+// whose tiles are partly empty does not lose (1000x60: 19.5 / 14.6 either way).
 // GK_STAGE_TILE overrides (tuning).
 int stage_tile_rows(const gk::Geom& g, int threads, int rows, bool parity) {
     const int forced = env_int("GK_STAGE_TILE", -1);

@@ -509,7 +509,7 @@ __device__ __forceinline__ double floors4_inv(double (&r)[4], const Phys& ph, De
 // q (a first stage: c1 = c2 = 1, no u0) and the flux difference dF, in the
 // reference's order: summing dF first, or q + c1 (u0 - q), saves an operation but
 // loses what the roundings make of c1 + c2 = 1 - 2^-54 in thirds (RT 1024x3072 after
-// 40 steps 1.3e-15 and 2.7e-15 from the 64-bit reference, 4.2e-16 in this order).
+// 40 steps 1.3e-15 and 2.7e-15 from the 64-bit reference, 4.6e-16 in this order).
 template <bool THREE>
 __device__ __forceinline__ double stage_value(double c1, double c2, double c3, double u0, double q,
                                               double dF) {
@@ -2216,7 +2216,9 @@ static inline int march_length(int n, int most, long long ctas, long long slots,
     return best;
 }
 // 3D stage: rows per CTA segment and the CTA width (64, 96 or 128 threads,
-// whichever wastes the fewest lanes on the last strip of columns).
+// whichever wastes the fewest lanes on the last strip of columns; at 64 / 96 / 128,
+// us per step: 92^3 fast 138 / 119 / 138, parity 247 / 206 / 247; 101x97x90 fast 154 /
+// 192 / 154, parity 267 / 354 / 268; 256^3 fast 2180 / 2130 / 2359, parity 3761 / 3672 / 4275).
 static inline int stage3d_rows(const Geom& g, int nt) {
     const long long strips = (g.nx + nt - 5) / (nt - 4);
     return march_length(g.ny, 32, strips * g.nz, 148LL * (kStage3dThreadsPerSM / nt), 2.5);

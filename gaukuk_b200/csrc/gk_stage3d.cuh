@@ -232,7 +232,7 @@ __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;
 // adiabatic.cpp:115-160, on the values it writes) and its last CTA runs the
 // step epilogue, as k_cfl would after it.
 // Resident threads per SM: 384, at up to 168 registers each (parity mode with
-// 40-72 bytes of spills).  Parity mode at 192^3: 1.74 ms per step, 1.72 at 256
+// 64-96 bytes of spills in 3D, 44-84 in 2D).  Parity mode at 192^3: 1.74 ms per step, 1.72 at 256
 // threads without spills, which loses 10-30 % on small grids (64^3: 158 us
 // against 207); fast mode at 512 threads (128 registers, no spills) is no faster
 // at 256^3 (2.175 -> 2.162 ms) and slower on small grids (31x190x55 82 -> 88 us).
